@@ -69,6 +69,7 @@ struct HostGeometry {
     std::vector<float> h_a, h_b;                                  // 4 floats per hole
     std::vector<int> h_plate;
     PlateBox plate[kMaxPlates];
+    float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};   // box of the crystals
 };
 
 // Parses and validates; returns SM_OK or an SM_ERR_* code with sm_last_error set.

@@ -40,6 +40,7 @@ struct PEParams {
     int n_sc, n_sv, group;   // sub-cells per crystal, sub-points per voxel, sub-points per mask group
     int pair;                // voxels per group of sub-points (1..8): > 1 when a voxel has at most 16 rays
     float inv_sv;
+    float chord_delta;       // half-size margin of chord_filter: 1.5e-6 of the coordinate range
     // reciprocals for the division-free index decode (exact after one correction step)
     float inv_n_sc, inv_dY, inv_dX, inv_kx, inv_ky, inv_kxky, inv_dXdY;
     int row0, row1;          // crystal rows [row0, row1)

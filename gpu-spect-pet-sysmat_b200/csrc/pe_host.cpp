@@ -61,6 +61,17 @@ void pe_plan(const HostGeometry& g, const int sv[3], const int sc[3], const int 
     }
     if (P.pair > 1) P.group = P.pair * P.n_sv;
     P.inv_sv = 1.0f / (float)P.n_sv;
+    // Range S of the coordinates a ray spans: the image (any rotation) and the crystals.
+    const float half[3] = {g.nx * g.voxel[0] * 0.5f + std::fabs(g.shift[0]), g.ny * g.voxel[1] * 0.5f + std::fabs(g.shift[1]),
+                           nz_full * g.voxel[2] * 0.5f + std::fabs(g.shift[2])};
+    const float round = std::sqrt(half[0] * half[0] + half[1] * half[1]);
+    float s2 = 0.0f;
+    for (int a = 0; a < 3; ++a) {
+        const float r = a < 2 ? round : half[2];
+        const float e = std::max(r, g.hi[a]) - std::min(-r, g.lo[a]);
+        s2 += e * e;
+    }
+    P.chord_delta = 1.5e-6f * std::sqrt(s2);
     P.inv_n_sc = 1.0f / (float)P.n_sc;
     P.inv_dY = 1.0f / (float)P.dY;
     P.inv_dX = 1.0f / (float)P.dX;

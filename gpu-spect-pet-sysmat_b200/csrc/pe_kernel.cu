@@ -58,8 +58,12 @@ constexpr float kMargin = 0.01f;     // mm added around every culling box
 constexpr float kConeMargin = 1e-5f; // float-filter band around the cone threshold
 constexpr int kPassSlots = 4;        // warp passes per group whose candidate masks are kept
 
+// List entry bit: every sub-point of the voxel passes the candidate's cone test.
+constexpr int kConeSure = 0x8000;
+static_assert(kSupC <= kConeSure && kSupH <= kConeSure, "staged-set indices share 16 bits with kConeSure");
+
 struct WarpLists {
-    unsigned short list_c[kListC];    // staged-set indices of the voxel's candidate crystals
+    unsigned short list_c[kListC];    // staged-set indices of the voxel's candidate crystals (kConeSure: see cone_sure)
     unsigned short list_h[kListH];    // ... and holes (ascending ids)
     unsigned short blist_c[kListC];   // staged-set indices the whole brick can reach for this warp's crystal
     unsigned short blist_h[kListH];   // (per-voxel lists narrow from these when they fit)
@@ -78,7 +82,7 @@ struct WarpLists {
 
 struct __align__(16) PeSmem {
     float4 c_pos[kSupC];     // cx, cy, cz, mu_total
-    float4 c_size[kSupC];    // w, t, h, crit
+    float4 c_half[kSupC];    // half sizes w/2, t/2, h/2 and the bounding radius crit/2 (all exact halves)
     float4 c_lo[kSupC];      // inflated world AABB (lower corner), cos(-rot)
     float4 c_hi[kSupC];      // ... (upper corner), sin(-rot)
     int c_id[kSupC];
@@ -139,7 +143,7 @@ __device__ __forceinline__ Vec3 subpoint_of(const PEParams& P, int ix, int iy, i
 
 // Per-crystal constants of the warp's detecting crystal.
 struct Detecting {
-    float cx, cy, cz, mu_t, mu_pe;
+    float cx, cy, cz, mu_t, pe_frac;   // pe_frac = mu_pe / mu_t
     float w, t, h, crit;
     float cm, sm, cp, sp;          // cos(-rot), sin(-rot), cos(rot), sin(rot)
     Box3 world;                    // inflated world AABB
@@ -197,6 +201,25 @@ __device__ __forceinline__ int cone_filter(const ConeSelf& cs, const Vec3& p, fl
     if (diff < -kConeMargin) return 1;
     if (diff > kConeMargin) return 0;
     return -1;
+}
+
+// True when every point p within rho of p0 passes the cone test of a candidate
+// (centre k, radius term rk / |k - p|) and the detecting crystal (centre d,
+// radius term rd / |d - p|).  With m a lower bound of both distances, the
+// difference of the unit vectors to k and d changes with p by at most
+// |1/|k-p| - 1/|d-p|| + 2 |u_k - u_d| / m <= 3 |k - d| / m^2 per unit length; the
+// 1e-4 is a hundred times the rounding of the test.
+__device__ __forceinline__ bool cone_sure(const Vec3& p0, float rho, float kx, float ky, float kz, float rk, float dx,
+                                          float dy, float dz, float rd) {
+    const float ax = kx - p0.x, ay = ky - p0.y, az = kz - p0.z, bx = dx - p0.x, by = dy - p0.y, bz = dz - p0.z;
+    const float a2 = fmaf(ax, ax, fmaf(ay, ay, az * az)), b2 = fmaf(bx, bx, fmaf(by, by, bz * bz));
+    const float ia = rsqrtf(a2), ib = rsqrtf(b2), da = a2 * ia, db = b2 * ib;
+    const float m = fminf(da, db) - rho;
+    const float ux = fmaf(ax, ia, -bx * ib), uy = fmaf(ay, ia, -by * ib), uz = fmaf(az, ia, -bz * ib);
+    const float lhs = sqrtf(fmaf(ux, ux, fmaf(uy, uy, uz * uz)));
+    const float cx = kx - dx, cy = ky - dy, cz = kz - dz;
+    const float grow = 3.0f * rho * sqrtf(fmaf(cx, cx, fmaf(cy, cy, cz * cz))) / (m * m);
+    return m > 1.0f && lhs + grow + 1e-4f <= rk / (da + rho) + rd / (db + rho);
 }
 
 __device__ __forceinline__ Box3 hole_box(const float4& a, const float4& b) {
@@ -262,6 +285,21 @@ __device__ __forceinline__ bool ray_may_hit(const RaySeg& r, const Box3& K) {
     const float za = fmaf(dz, lmin, r.p.z), zb = fmaf(dz, lmax, r.p.z);
     if (fminf(za, zb) > K.z2 || fmaxf(za, zb) < K.z1) return false;
     return true;
+}
+
+// The reference's exact chords out of line: taken only where the filters cannot call.
+__device__ __noinline__ float crystal_chord_exact(Vec3 p, Vec3 q, float4 kp, float4 kh, float kc, float ks) {
+    const float yIa = p.y - kp.y;
+    const float yDa = q.y - kp.y;
+    const float xIa = (p.x - kp.x) * kc - (p.z - kp.z) * ks;
+    const float zIa = (p.x - kp.x) * ks + (p.z - kp.z) * kc;
+    const float xDa = (q.x - kp.x) * kc - (q.z - kp.z) * ks;
+    const float zDa = (q.x - kp.x) * ks + (q.z - kp.z) * kc;
+    return chord_through(xIa, yIa, zIa, xDa, yDa, zDa, Box3{-kh.x, -kh.y, -kh.z, kh.x, kh.y, kh.z});
+}
+
+__device__ __noinline__ float hole_chord_exact(Vec3 p, Vec3 q, float4 ha, float R) {
+    return chord_hole(p.x, p.y, p.z, q.x, q.y, q.z, ha.x, ha.y, ha.z, ha.w, R);
 }
 
 // Exact plate test out of line (rarely needed: see plate_traversed).
@@ -332,7 +370,7 @@ __device__ __forceinline__ float ray_value(const Detecting& D, const Vec3& ps, f
     }
     att = fmaf(self_len, D.mu_t, att);
     const float eff = __expf(-att);
-    const float absorb = (1.0f - __expf(-absorb_len * D.mu_t)) * D.mu_pe / D.mu_t;
+    const float absorb = (1.0f - __expf(-absorb_len * D.mu_t)) * D.pe_frac;
     // Solid angle: the largest of the three projected sub-cell faces (:618-639),
     // A * |cos| / (4 pi d^2).
     const float k4 = 0.0795774715459476678f * inv_r * inv_r * inv_r;   // 1 / (4 pi d^3)
@@ -395,6 +433,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
     const float dsq = fmaf(dy, dy, fmaf(dxw, dxw, dzw * dzw));
     const float inv_r = rsqrtf(dsq);
     const float r = dsq * inv_r;
+    const ChordRay cr = make_chord_ray(p.x, p.y, p.z, dxw, dy, dzw, r);
 
     int rec_h = 0, rec_c = 0;
     float att = 0.0f;
@@ -411,18 +450,22 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             while (bits) {
                 const int b = __ffs(bits) - 1;
                 bits &= bits - 1;
-                const int k = L.list_h[(wd << 5) + b];
+                const int e = L.list_h[(wd << 5) + b], k = e & (kConeSure - 1);
                 const float4 ha = S.h_a[k], hbv = S.h_b[k];
-                if (!ray_may_hit(seg, hole_box(ha, hbv))) continue;
+                if (dy > 0.0f && p.y < ha.y &&
+                    hole_missed(p.x, p.y, p.z, dxw, dzw, cr.iy, ha.x, ha.y, ha.z, ha.w, hbv.x, kMargin))
+                    continue;
                 if (n_hole) ++*n_hole;
-                const float len = chord_hole(p.x, p.y, p.z, q.x, q.y, q.z, ha.x, ha.y, ha.z, ha.w, hbv.x);
+                const float len = hole_chord_exact(p, q, ha, hbv.x);
                 if (len == 0.0f) continue;
-                if (n_cone) ++*n_cone;
-                const float4 c4 = *csp;
-                const ConeSelf cs{c4.x, c4.y, c4.z, c4.w};
-                int f = cone_filter(cs, p, ha.x, hbv.w, ha.w, hbv.z);
-                if (f < 0) f = cone_hole_exact(cs, p, ha.x, hbv.w, ha.w, hbv.z) ? 1 : 0;
-                if (!f) continue;
+                if (!(e & kConeSure)) {
+                    if (n_cone) ++*n_cone;
+                    const float4 c4 = *csp;
+                    const ConeSelf cs{c4.x, c4.y, c4.z, c4.w};
+                    int f = cone_filter(cs, p, ha.x, hbv.w, ha.w, hbv.z);
+                    if (f < 0) f = cone_hole_exact(cs, p, ha.x, hbv.w, ha.w, hbv.z) ? 1 : 0;
+                    if (!f) continue;
+                }
                 in_holes += len;
                 att += hbv.y * len;
                 if (RECORD && len > 0.0f) {
@@ -443,40 +486,34 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
         while (bits) {
             const int b = __ffs(bits) - 1;
             bits &= bits - 1;
-            const int k = L.list_c[(wd << 5) + b];
-            const float4 klo = S.c_lo[k], khi = S.c_hi[k];
-            if (!ray_may_hit(seg, box_of(klo, khi))) continue;
-            if (n_cry) ++*n_cry;
-            const float4 kp = S.c_pos[k], ks = S.c_size[k];
-            const float2 kr = make_float2(klo.w, khi.w);
-            const float yIa = p.y - kp.y;
-            const float yDa = q.y - kp.y;
-            float xIa, zIa, xDa, zDa;
-            if (kr.x == 1.0f && kr.y == 0.0f) {
-                // Unrotated crystal: a * 1 - b * (+-0) and a * (+-0) + b * 1
-                // round to a and b exactly.  Only the sign of a zero result
-                // can differ, and chord_through never divides by a coordinate:
-                // it subtracts them from nonzero box bounds, compares them, and
-                // divides only by differences of at least 0.001.
-                xIa = p.x - kp.x;
-                zIa = p.z - kp.z;
-                xDa = q.x - kp.x;
-                zDa = q.z - kp.z;
+            const int e = L.list_c[(wd << 5) + b], k = e & (kConeSure - 1);
+            const float4 kp = S.c_pos[k], kh = S.c_half[k];
+            const float kc = S.c_lo[k].w, ks = S.c_hi[k].w;   // cos, sin of the crystal's rotation
+            float len = 0.0f;
+            int f;
+            if (kc == 1.0f && ks == 0.0f) {
+                f = chord_filter(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, P.chord_delta, &len);
             } else {
-                xIa = (p.x - kp.x) * kr.x - (p.z - kp.z) * kr.y;
-                zIa = (p.x - kp.x) * kr.y + (p.z - kp.z) * kr.x;
-                xDa = (q.x - kp.x) * kr.x - (q.z - kp.z) * kr.y;
-                zDa = (q.x - kp.x) * kr.y + (q.z - kp.z) * kr.x;
+                // the segment in the crystal's frame; its rotation rounds once more, hence twice the margin
+                const float px = p.x - kp.x, pz = p.z - kp.z;
+                const ChordRay kr = make_chord_ray(fmaf(px, kc, -pz * ks), p.y - kp.y, fmaf(px, ks, pz * kc),
+                                                   fmaf(dxw, kc, -dzw * ks), dy, fmaf(dxw, ks, dzw * kc), r);
+                f = kr.ok ? chord_filter(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, 2.0f * P.chord_delta, &len) : -1;
             }
-            const Box3 kb{-0.5f * ks.x, -0.5f * ks.y, -0.5f * ks.z, 0.5f * ks.x, 0.5f * ks.y, 0.5f * ks.z};
-            const float len = chord_through(xIa, yIa, zIa, xDa, yDa, zDa, kb);
-            if (len == 0.0f) continue;
-            if (n_cone) ++*n_cone;
-            const float4 c4 = *csp;
-            const ConeSelf cs{c4.x, c4.y, c4.z, c4.w};
-            int f = cone_filter(cs, p, kp.x, kp.y, kp.z, 0.5f * ks.w);
-            if (f < 0) f = cone_crystal_exact(cs, p, kp.x, kp.y, kp.z, ks.w) ? 1 : 0;
+            if (n_cry && f) ++*n_cry;
+            if (f < 0 || !cr.ok) {
+                len = crystal_chord_exact(p, q, kp, kh, kc, ks);
+                f = len != 0.0f;
+            }
             if (!f) continue;
+            if (!(e & kConeSure)) {
+                if (n_cone) ++*n_cone;
+                const float4 c4 = *csp;
+                const ConeSelf cs{c4.x, c4.y, c4.z, c4.w};
+                int g = cone_filter(cs, p, kp.x, kp.y, kp.z, kh.w);
+                if (g < 0) g = cone_crystal_exact(cs, p, kp.x, kp.y, kp.z, 2.0f * kh.w) ? 1 : 0;
+                if (!g) continue;
+            }
             att += len * kp.w;
             if (RECORD && len > 0.0f) {
                 if (rec_c < kRecCrystals) rec[3 + kRecHoles + rec_c] = S.c_id[k];
@@ -716,7 +753,8 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
         if (pass) {
             if (off < kSupC) {
                 S.c_pos[off] = G.c.pos[k];
-                S.c_size[off] = G.c.size[k];
+                const float4 sz = G.c.size[k];
+                S.c_half[off] = make_float4(0.5f * sz.x, 0.5f * sz.y, 0.5f * sz.z, 0.5f * sz.w);
                 const float4 rr = G.c.rot[k];
                 S.c_lo[off] = make_float4(lo.x - kMargin, lo.y - kMargin, lo.z - kMargin, rr.x);
                 S.c_hi[off] = make_float4(hi.x + kMargin, hi.y + kMargin, hi.z + kMargin, rr.y);
@@ -775,7 +813,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
         Detecting D;
         {
             const float4 pos = G.c.pos[d], sz = G.c.size[d], rt = G.c.rot[d], ph = G.c.phys[d];
-            D.cx = pos.x; D.cy = pos.y; D.cz = pos.z; D.mu_t = pos.w; D.mu_pe = ph.x;
+            D.cx = pos.x; D.cy = pos.y; D.cz = pos.z; D.mu_t = pos.w; D.pe_frac = ph.x / pos.w;
             D.w = sz.x; D.t = sz.y; D.h = sz.z; D.crit = sz.w;
             D.cm = rt.x; D.sm = rt.y; D.cp = rt.z; D.sp = rt.w;
             D.world = S.d_box[warp];
@@ -820,6 +858,9 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
         // (P.pair, up to 8): a pass then traces one sub-cell column from all of
         // them, and the lanes of each voxel are summed apart.
         const int VP = RECORD ? 1 : P.pair;
+        // Flagging the candidates that surely pass the cone test pays once a voxel's
+        // lists serve four passes or more (one pass per list: 7 % slower with it).
+        const bool flag_sure = P.pair == 1 && P.n_sv * P.n_sc >= 128;
         for (int vl = 0; vl < tv; vl += VP) {
             // voxel u of the group is brick voxel vl + u
             auto vox_of = [&](int u, int& x, int& y, int& z) {
@@ -859,6 +900,9 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                 bool slow = S.overflow != 0;
                 if (!slow) {
                     const Bundle bv = make_bundle(Avox, D.world);
+                    const Vec3 mid{0.5f * (Avox.x1 + Avox.x2), 0.5f * (Avox.y1 + Avox.y2), 0.5f * (Avox.z1 + Avox.z2)};
+                    const float ex = Avox.x2 - mid.x, ey = Avox.y2 - mid.y, ez = Avox.z2 - mid.z;
+                    const float rho = sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
                     int cnt = 0;
                     const int src_c = brick ? L.nb_c : n_c;
                     for (int i0 = 0; i0 < src_c; i0 += 32) {
@@ -868,6 +912,9 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                         if (i < src_c) {
                             k = brick ? (int)L.blist_c[i] : i;
                             pass = (brick || S.c_id[k] != d) && bundle_hit(bv, box_of(S.c_lo[k], S.c_hi[k]));
+                            const float4 kp = S.c_pos[k];
+                            if (pass && flag_sure && cone_sure(mid, rho, kp.x, kp.y, kp.z, S.c_half[k].w, D.cx, D.cy, D.cz, 0.5f * D.crit))
+                                k |= kConeSure;
                         }
                         cnt = warp_append(pass, k, L.list_c, cnt, kListC, lane);
                     }
@@ -879,7 +926,10 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                         bool pass = false;
                         if (i < src_h) {
                             k = brick ? (int)L.blist_h[i] : i;
-                            pass = bundle_hit(bv, hole_box(S.h_a[k], S.h_b[k]));
+                            const float4 ha = S.h_a[k], hb = S.h_b[k];
+                            pass = bundle_hit(bv, hole_box(ha, hb));
+                            if (pass && flag_sure && cone_sure(mid, rho, ha.x, hb.w, ha.w, hb.z, D.cx, D.cy, D.cz, 0.5f * D.crit))
+                                k |= kConeSure;
                         }
                         cnth = warp_append(pass, k, L.list_h, cnth, kListH, lane);
                     }
@@ -893,7 +943,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                         int below = 0;
                         for (int i0 = 0; i0 < cnth; i0 += 32) {
                             const int i = i0 + lane;
-                            below += __popc(__ballot_sync(0xffffffffu, i < cnth && S.h_id[L.list_h[i]] < first));
+                            below += __popc(__ballot_sync(0xffffffffu, i < cnth && S.h_id[L.list_h[i] & (kConeSure - 1)] < first));
                         }
                         if (lane == 0) L.plate_begin[m] = below;
                     }
@@ -998,7 +1048,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                             for (int w = 0; w < nwc; ++w) {
                                 bool pass = false;
                                 if ((w << 5) + lane < lc) {
-                                    const int k = L.list_c[(w << 5) + lane];
+                                    const int k = L.list_c[(w << 5) + lane] & (kConeSure - 1);
                                     pass = bundle_hit(bq, box_of(S.c_lo[k], S.c_hi[k]));
                                 }
                                 const unsigned bal = __ballot_sync(0xffffffffu, pass);
@@ -1007,7 +1057,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                             for (int w = 0; w < nwh; ++w) {
                                 bool pass = false;
                                 if ((w << 5) + lane < lh) {
-                                    const int k = L.list_h[(w << 5) + lane];
+                                    const int k = L.list_h[(w << 5) + lane] & (kConeSure - 1);
                                     pass = bundle_hit(bq, hole_box(S.h_a[k], S.h_b[k]));
                                 }
                                 const unsigned bal = __ballot_sync(0xffffffffu, pass);

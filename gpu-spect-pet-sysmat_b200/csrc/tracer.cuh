@@ -215,6 +215,83 @@ SM_HD float chord_hole(float xi, float yi, float zi, float xo, float yo, float z
     return (float)((double)t_b - r1);
 }
 
+// ---- chord_through decided without its divisions and square root -----------------
+// A segment a -> b prepared once for many boxes: its start, the reciprocal of
+// its extent on each axis and their magnitudes, its length.
+struct ChordRay {
+    float px, py, pz;
+    float ix, iy, iz, ax, ay, az;
+    float len;
+    bool ok;      // no axis is near the reference's degenerate extent (0.001)
+};
+
+// 1 / d to about one unit in the last place.
+SM_HD float chord_rcp(float d) {
+#ifdef __CUDA_ARCH__
+    const float r = __fdividef(1.0f, d);
+#else
+    const float r = 1.0f / d;
+#endif
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
+
+SM_HD ChordRay make_chord_ray(float px, float py, float pz, float dx, float dy, float dz, float len) {
+    ChordRay c;
+    c.px = px; c.py = py; c.pz = pz;
+    c.ix = chord_rcp(dx); c.iy = chord_rcp(dy); c.iz = chord_rcp(dz);
+    c.ax = fabsf(c.ix); c.ay = fabsf(c.iy); c.az = fabsf(c.iz);
+    c.len = len;
+    c.ok = fminf(fminf(fabsf(dx), fabsf(dy)), fabsf(dz)) > 0.002f;
+    return c;
+}
+
+// chord_through of the box of half sizes (hx, hy, hz) about (cx, cy, cz), when
+// the answer is clear: 1 (the chord, in `chord`), 0 (no chord) or -1 (too
+// close to call: chord_through decides).  In units of the segment, axis i of
+// the box grown or shrunk by delta is crossed between t_i -+ (h_i +- delta) |1/d_i|;
+// `grown` bounds the reference's tmin from below and its tmax from above,
+// `shrunk` the other way round, so a condition that both satisfy is the
+// reference's.  delta covers the rounding of either form: the boxes' corners
+// in the segment's frame (2 units of 2^-24 of the coordinate range S), and the
+// slab parameters along the segment (10 units of its length <= S), together
+// below 8e-7 S; pe_plan passes 1.5e-6 S.
+SM_HD int chord_filter(const ChordRay& r, float cx, float cy, float cz, float hx, float hy, float hz, float delta,
+                       float* chord) {
+    const float eps = 0.001f;
+    const float tx = (cx - r.px) * r.ix, ty = (cy - r.py) * r.iy, tz = (cz - r.pz) * r.iz;
+    const float gx = hx + delta, gy = hy + delta, gz = hz + delta;
+    const float sx = hx - delta, sy = hy - delta, sz = hz - delta;
+    const float lo_g = fmaxf(fmaxf(fmaf(-gx, r.ax, tx), fmaf(-gy, r.ay, ty)), fmaf(-gz, r.az, tz));
+    const float hi_g = fminf(fminf(fmaf(gx, r.ax, tx), fmaf(gy, r.ay, ty)), fmaf(gz, r.az, tz));
+    const float lo_s = fmaxf(fmaxf(fmaf(-sx, r.ax, tx), fmaf(-sy, r.ay, ty)), fmaf(-sz, r.az, tz));
+    const float hi_s = fminf(fminf(fmaf(sx, r.ax, tx), fmaf(sy, r.ay, ty)), fmaf(sz, r.az, tz));
+    if ((hi_g - lo_g) * r.len < eps || hi_s > 1.0f || lo_s * r.len < eps) return 0;
+    if ((hi_s - lo_s) * r.len > eps && hi_g < 1.0f && lo_g * r.len > eps) {
+        const float lo = fmaxf(fmaxf(fmaf(-hx, r.ax, tx), fmaf(-hy, r.ay, ty)), fmaf(-hz, r.az, tz));
+        const float hi = fminf(fminf(fmaf(hx, r.ax, tx), fmaf(hy, r.ay, ty)), fmaf(hz, r.az, tz));
+        *chord = (hi - lo) * r.len;
+        return 1;
+    }
+    return -1;
+}
+
+// True when the segment a -> b (inv_dy = 1 / (b_y - a_y)) surely misses the hole
+// cylinder: between the depth planes y1, y2 its lateral distance to the axis stays
+// above R + margin.  Valid for segments that run towards larger y.
+SM_HD bool hole_missed(float px, float py, float pz, float dx, float dz, float inv_dy, float xc, float y1, float y2,
+                       float zc, float R, float margin) {
+    const float l1 = (y1 - py) * inv_dy, l2 = (y2 - py) * inv_dy;
+    const float wx = xc - fmaf(dx, l1, px), wz = zc - fmaf(dz, l1, pz);
+    const float ex = dx * (l2 - l1), ez = dz * (l2 - l1);
+    const float ee = fmaf(ex, ex, ez * ez), we = fmaf(wx, ex, wz * ez);
+    const float reach = R + margin, r2 = reach * reach;
+    const float ww = fmaf(wx, wx, wz * wz);
+    if (we <= 0.0f) return ww > r2;                                   // nearest at the y1 plane
+    if (we >= ee) return ww - 2.0f * we + ee > r2;                    // ... at the y2 plane
+    const float cr = fmaf(wx, ez, -wz * ex);
+    return cr * cr > r2 * ee;
+}
+
 // Conservative culling: can any segment from a point of box A to a point of
 // box B meet box K?  K must already be inflated by the safety margin.  Uses
 // the depth (y) ordering of the scanner: at depth y a segment a -> b sits at

@@ -1,0 +1,80 @@
+// Compares the tracer's chord_filter and hole_missed with the reference-order
+// chord_through and chord_hole on the host: chord_filter_check SEED COUNT RANGE.
+// Prints "<wrong calls> <clear hits> <clear misses> <unclear> <largest value error>".
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+
+#include "tracer.cuh"
+
+using namespace smb;
+
+int main(int argc, char** argv) {
+    if (argc < 4) return 2;
+    std::mt19937_64 gen(std::strtoull(argv[1], nullptr, 10));
+    const long n = std::atol(argv[2]);
+    const float range = (float)std::atof(argv[3]), delta = 1.5e-6f * range;
+    auto U = [&](float a, float b) { return std::uniform_real_distribution<float>(a, b)(gen); };
+    auto side = [&](float h) { return U(0, 1) < 0.5f ? -h : h; };
+    const float lat = 0.35f * range;   // image and detector half width; depth up to half the range
+    long wrong = 0, hits = 0, misses = 0, unclear = 0;
+    double worst = 0.0;
+    for (long i = 0; i < n; ++i) {
+        const float hx = U(0.3f, 2), hy = U(0.3f, 4), hz = U(0.3f, 2), near = 3 * delta;
+        const float ky = U(0.25f, 0.45f) * range;
+        float px = U(-lat, lat), py = U(-0.2f, 0.1f) * range, pz = U(-lat, lat);
+        float qx = U(-lat, lat), qy = ky + U(-hy, 3 * hy), qz = U(-lat, lat);
+        // the box: around the ray, or with an edge or a corner within a few margins of it
+        const float depth = ky + (i % 4 < 2 ? side(hy) : U(-hy, hy)), l = (depth - py) / (qy - py);
+        float kx = px + (qx - px) * l, kz = pz + (qz - pz) * l;
+        if (i & 1) {
+            kx += U(-1.5f, 1.5f) * hx;
+            kz += U(-1.5f, 1.5f) * hz;
+        } else {
+            kx += side(hx) + U(-near, near);
+            kz += U(0, 1) < 0.3f ? U(-hz, hz) : side(hz) + U(-near, near);
+        }
+        if (i % 7 == 0) {          // the segment ends at the box's faces
+            qx = kx + U(-1.2f, 1.2f) * hx;
+            qz = kz + U(-1.2f, 1.2f) * hz;
+            qy = ky + side(hy) + U(-0.003f, 0.003f);
+        }
+        if (i % 11 == 0) px = qx + U(-0.004f, 0.004f);       // nearly parallel to a face
+        if (i % 13 == 0) {         // ... or starts there
+            px = kx + side(hx) + U(-0.002f, 0.002f);
+            py = ky - hy + U(-0.003f, 0.003f);
+            pz = kz + U(-1, 1) * hz;
+        }
+        const float dx = qx - px, dy = qy - py, dz = qz - pz, len = std::sqrt(dx * dx + dy * dy + dz * dz);
+        const ChordRay r = make_chord_ray(px, py, pz, dx, dy, dz, len);
+        const Box3 box{-hx, -hy, -hz, hx, hy, hz};
+        float chord = 0, ref;
+        int f;
+        if (i % 3) {
+            f = r.ok ? chord_filter(r, kx, ky, kz, hx, hy, hz, delta, &chord) : -1;
+            ref = chord_through(px - kx, py - ky, pz - kz, qx - kx, qy - ky, qz - kz, box);
+        } else {
+            const float a = U(-0.5f, 0.5f), c = std::cos(a), s = std::sin(a), ax = px - kx, az = pz - kz;
+            const ChordRay k = make_chord_ray(fmaf(ax, c, -az * s), py - ky, fmaf(ax, s, az * c), fmaf(dx, c, -dz * s), dy,
+                                              fmaf(dx, s, dz * c), len);
+            f = k.ok ? chord_filter(k, 0, 0, 0, hx, hy, hz, 2 * delta, &chord) : -1;
+            ref = chord_through(ax * c - az * s, py - ky, ax * s + az * c, (qx - kx) * c - (qz - kz) * s, qy - ky,
+                                (qx - kx) * s + (qz - kz) * c, box);
+        }
+        if (f < 0) ++unclear;
+        else if (f == 0) { ++misses; wrong += ref != 0; }
+        else {
+            ++hits;
+            wrong += ref == 0;
+            worst = std::fmax(worst, std::fabs((double)chord - ref) / (delta * len * std::fmax(r.ax, std::fmax(r.ay, r.az))));
+        }
+        // a hole of radius hx between ky - hy and ky + hy
+        if (py < ky - hy && dy > 0 &&
+            hole_missed(px, py, pz, dx, dz, r.iy, kx, ky - hy, ky + hy, kz, hx, 0.01f) &&
+            chord_hole(px, py, pz, qx, qy, qz, kx, ky - hy, ky + hy, kz, hx) != 0)
+            ++wrong;
+    }
+    std::printf("%ld %ld %ld %ld %.3g\n", wrong, hits, misses, unclear, worst);
+    return 0;
+}
