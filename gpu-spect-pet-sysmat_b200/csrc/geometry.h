@@ -72,6 +72,14 @@ struct HostGeometry {
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};   // box of the crystals
 };
 
+// Grows the crystals' box by crystal d's.
+inline void add_crystal_box(HostGeometry* g, int d, const float lo[3], const float hi[3]) {
+    for (int a = 0; a < 3; ++a) {
+        if (d == 0 || lo[a] < g->lo[a]) g->lo[a] = lo[a];
+        if (d == 0 || hi[a] > g->hi[a]) g->hi[a] = hi[a];
+    }
+}
+
 // Parses and validates; returns SM_OK or an SM_ERR_* code with sm_last_error set.
 int parse_geometry(const float* col, size_t n_col, const float* det, size_t n_det, const float* img,
                    size_t n_img, const float* phy, size_t n_phy, HostGeometry* out);

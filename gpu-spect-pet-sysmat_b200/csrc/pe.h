@@ -38,11 +38,11 @@ struct PEParams {
     float cos_a, sin_a;      // image rotation about z
     int dX, dY, dZ;          // crystal sub-cells
     int n_sc, n_sv, group;   // sub-cells per crystal, sub-points per voxel, sub-points per mask group
-    int pair;                // voxels per group of sub-points (1..8): > 1 when a voxel has at most 16 rays
+    int pair;                // voxels per group of sub-points (1..8): > 1 for entries of at most 64 rays (see pe_plan)
     float inv_sv;
     float chord_delta;       // half-size margin of chord_filter: 1.5e-6 of the coordinate range
     // reciprocals for the division-free index decode (exact after one correction step)
-    float inv_n_sc, inv_dY, inv_dX, inv_kx, inv_ky, inv_kxky, inv_dXdY;
+    float inv_n_sc, inv_n_sv, inv_dY, inv_dX, inv_kx, inv_ky, inv_kxky, inv_dXdY, inv_bx, inv_bxy;
     int row0, row1;          // crystal rows [row0, row1)
     int bx, by, bz;          // voxel brick
     int tiles_x, tiles_y, tiles_z;
@@ -68,9 +68,13 @@ struct PEParams {
 // rays are ordered (sub-cell column, sub-point, depth sub-cell) and dealt to
 // the lanes in order; the group changes which lane sums which ray (the
 // rounding of the sums), never a hit decision.
+// slots: CTAs the device holds at once when the plan is launched by itself (the
+// default brick then shrinks until the launch fills them), 0 when its tiles
+// join others' in a batch.
 void pe_plan(const HostGeometry& g, const int sv[3], const int sc[3], const int brick[3], int group, int rotation,
-             int row0, int row1, int nz_full, int z0, int nz, PEParams* p);
+             int row0, int row1, int nz_full, int z0, int nz, int slots, PEParams* p);
 int pe_auto_group(int depth_subcells);
+inline int pe_slots(int sm_count) { return 2 * sm_count; }   // CTAs resident at once (the kernel's launch bound)
 
 // Launches the trace kernel (RECORD selects the hit-recording instantiation).
 cudaError_t pe_launch(const PEParams& p, const DevGeometry& geo, bool record, long long n_tiles, cudaStream_t stream);

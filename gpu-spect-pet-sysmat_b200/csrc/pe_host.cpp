@@ -12,7 +12,7 @@ namespace smb {
 int pe_auto_group(int depth_subcells) { return std::max(1, std::min(kMaxGroup, 32 / std::max(1, depth_subcells))); }
 
 void pe_plan(const HostGeometry& g, const int sv[3], const int sc[3], const int brick[3], int group, int rotation,
-             int row0, int row1, int nz_full, int z0, int nz, PEParams* p) {
+             int row0, int row1, int nz_full, int z0, int nz, int slots, PEParams* p) {
     PEParams& P = *p;
     P = PEParams();
     P.nx = g.nx;
@@ -44,19 +44,19 @@ void pe_plan(const HostGeometry& g, const int sv[3], const int sc[3], const int 
     P.n_sc = sc[0] * sc[1] * sc[2];
     P.n_sv = sv[0] * sv[1] * sv[2];
     P.group = group > 0 ? std::min(group, kMaxGroup) : pe_auto_group(P.dY);
-    // Entries of at most 16 rays: VP neighbouring voxels form one group of
-    // sub-points (VP * n_sv <= kMaxGroup), so that a warp pass traces one
-    // sub-cell column from all of them.  The kernel sums each lane's rays for
-    // one voxel, so the lane-to-point map must be the same in every pass: the
-    // group's rays fit one pass, or a sub-cell column's rays (cb) divide 32.
+    // Entries of at most 64 rays whose sub-points are fewer than a group: VP
+    // neighbouring voxels form one group (VP * n_sv <= kMaxGroup), so that a warp
+    // pass traces one sub-cell column from all of them and one set of lists serves
+    // them (2.1x on 64-ray entries; entries of 1024 sub-cells, whose own passes
+    // amortise the lists, ran 8 % slower in pairs of voxels).  The kernel sums each lane's rays for one voxel, so
+    // the lane-to-point map must be the same in every pass: the group's rays fit
+    // one pass, or a sub-cell column's rays (cb) divide 32.
     P.pair = 1;
-    if (P.n_sv * P.n_sc <= 16) {
-        for (int vp = 8; vp >= 2; vp >>= 1) {
-            const int g = vp * P.n_sv, cb = g * P.dY;
-            if (g <= kMaxGroup && (g * P.n_sc <= 32 || (cb <= 32 && 32 % cb == 0))) {
-                P.pair = vp;
-                break;
-            }
+    for (int vp = P.n_sv * P.n_sc <= 64 ? 8 : 1; vp >= 2; vp >>= 1) {
+        const int g = vp * P.n_sv, cb = g * P.dY;
+        if (g <= kMaxGroup && (g * P.n_sc <= 32 || (cb <= 32 && 32 % cb == 0))) {
+            P.pair = vp;
+            break;
         }
     }
     if (P.pair > 1) P.group = P.pair * P.n_sv;
@@ -73,6 +73,7 @@ void pe_plan(const HostGeometry& g, const int sv[3], const int sc[3], const int 
     }
     P.chord_delta = 1.5e-6f * std::sqrt(s2);
     P.inv_n_sc = 1.0f / (float)P.n_sc;
+    P.inv_n_sv = 1.0f / (float)P.n_sv;
     P.inv_dY = 1.0f / (float)P.dY;
     P.inv_dX = 1.0f / (float)P.dX;
     P.inv_kx = 1.0f / (float)P.kx;
@@ -92,13 +93,29 @@ void pe_plan(const HostGeometry& g, const int sv[3], const int sc[3], const int 
         else if (by >= bx && by > 1) by = (by + 1) / 2;
         else bx = (bx + 1) / 2;
     }
+    // A launch of few tiles: smaller bricks until the tiles fill the device once,
+    // down to one group of voxels; on to sixteen waves (a short last wave) while a
+    // warp keeps at least 64 passes per tile, against which the tile's cull is small.
+    const int n_ctiles = (row1 - row0 + kPeWarps - 1) / kPeWarps;
+    auto tiles = [&] {
+        return (long long)n_ctiles * ((g.nx + bx - 1) / bx) * ((g.ny + by - 1) / by) * ((nz + bz - 1) / bz);
+    };
+    while (slots > 0 && brick[0] <= 0 && brick[1] <= 0 && brick[2] <= 0 && bx * by * bz > P.pair) {
+        const long long t = tiles(), passes = (long long)bx * by * bz * P.n_sv * P.n_sc / 32;
+        if (t >= 16LL * slots || (t >= slots && passes < 128)) break;
+        if (bz > 1) bz = (bz + 1) / 2;
+        else if (by > 1) by = (by + 1) / 2;
+        else bx = (bx + 1) / 2;
+    }
     P.bx = bx;
     P.by = by;
     P.bz = bz;
+    P.inv_bx = 1.0f / (float)bx;
+    P.inv_bxy = 1.0f / (float)(bx * by);
     P.tiles_x = (g.nx + bx - 1) / bx;
     P.tiles_y = (g.ny + by - 1) / by;
     P.tiles_z = (nz + bz - 1) / bz;
-    P.n_ctiles = (row1 - row0 + kPeWarps - 1) / kPeWarps;
+    P.n_ctiles = n_ctiles;
     P.n_tiles = (long long)P.n_ctiles * P.tiles_x * P.tiles_y * P.tiles_z;
 }
 

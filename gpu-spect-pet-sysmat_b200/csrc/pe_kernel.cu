@@ -56,11 +56,24 @@ constexpr int kLWC = kListC / 32;
 constexpr int kLWH = kListH / 32;
 constexpr float kMargin = 0.01f;     // mm added around every culling box
 constexpr float kConeMargin = 1e-5f; // float-filter band around the cone threshold
-constexpr int kPassSlots = 4;        // warp passes per group whose candidate masks are kept
+constexpr int kColTable = 4;         // sub-cell columns of the crystal whose centres are kept
 
-// List entry bit: every sub-point of the voxel passes the candidate's cone test.
-constexpr int kConeSure = 0x8000;
-static_assert(kSupC <= kConeSure && kSupH <= kConeSure, "staged-set indices share 16 bits with kConeSure");
+// List entry: a staged-set index and two flags.
+constexpr int kConeSure = 0x8000;   // every sub-point of the voxel passes the candidate's cone test
+constexpr int kRotated = 0x4000;    // the crystal is rotated
+constexpr int kIndex = 0x3fff;
+static_assert(kSupC <= kIndex && kSupH <= kIndex, "staged-set indices share 16 bits with the flags");
+
+// Per-crystal constants of the warp's detecting crystal.
+struct Detecting {
+    float cx, cy, cz, mu_t, pe_frac;   // pe_frac = mu_pe / mu_t
+    float w, t, h, crit;
+    float cm, sm, cp, sp;          // cos(-rot), sin(-rot), cos(rot), sin(rot)
+    Box3 world;                    // inflated world AABB
+    float area_x, area_z, area_y;  // sub-cell face areas (t*h/dZ/dY, w*t/dX/dY, w*h/dX/dZ)
+    float hx, hy, hz;              // sub-cell half sizes
+    bool rotated;
+};
 
 struct WarpLists {
     unsigned short list_c[kListC];    // staged-set indices of the voxel's candidate crystals (kConeSure: see cone_sure)
@@ -70,14 +83,11 @@ struct WarpLists {
     int n_c, n_h;
     int nb_c, nb_h;
     int plate_begin[kMaxPlates + 1];  // list_h index where each plate's holes start
-    float4 cs[kMaxGroup];             // per sub-point of the group: the detecting crystal's cone (ConeSelf)
-    float4 pt[kMaxGroup];             // ... the sub-point in the world
-    float4 pself[kMaxGroup];          // ... and in the detecting crystal's frame
-    // Per warp pass: the candidates the pass's bundle of rays can reach.  Slot
-    // i holds pass i of a group; full groups of one voxel trace the same
-    // sub-cells in the same passes, so later groups reuse the first one's.
-    unsigned pass_c[kPassSlots][kLWC];
-    unsigned pass_h[kPassSlots][kLWH];
+    float4 cs[kMaxGroup];             // groups of several voxels, per point: the detecting crystal's cone (ConeSelf)
+    float4 pt[kMaxGroup];             // ... the point in the world
+    Detecting det;                    // in shared memory: its fields would take 25 registers of the tracing loop
+    float4 col[kColTable];            // per sub-cell column: centre x, z in the crystal's frame, then in the world
+    unsigned pass_c[kLWC], pass_h[kLWH];   // the candidates the current pass's bundle of rays can reach
 };
 
 struct __align__(16) PeSmem {
@@ -141,16 +151,6 @@ __device__ __forceinline__ Vec3 subpoint_of(const PEParams& P, int ix, int iy, i
     return subpoint(P, ix * P.kx + sx, iy * P.ky + sy, iz * P.kz + sz);
 }
 
-// Per-crystal constants of the warp's detecting crystal.
-struct Detecting {
-    float cx, cy, cz, mu_t, pe_frac;   // pe_frac = mu_pe / mu_t
-    float w, t, h, crit;
-    float cm, sm, cp, sp;          // cos(-rot), sin(-rot), cos(rot), sin(rot)
-    Box3 world;                    // inflated world AABB
-    float area_x, area_z, area_y;  // sub-cell face areas (t*h/dZ/dY, w*t/dX/dY, w*h/dX/dZ)
-    float hx, hy, hz;              // sub-cell half sizes
-};
-
 // ---- candidate cone test (PESysMatGen.cu:506-589) -----------------------------
 struct ConeSelf {
     float ux, uy, uz, crit_self;
@@ -164,6 +164,13 @@ __device__ __forceinline__ ConeSelf cone_self(const Detecting& D, const Vec3& p)
     c.uy = (D.cy - p.y) / dist;
     c.uz = (D.cz - p.z) / dist;
     return c;
+}
+
+// The group's table when there is one, else computed for this ray (few rays need it then: see kConeSure).
+__device__ __forceinline__ ConeSelf cone_of(const float4* table, const Detecting& D, const Vec3& p) {
+    if (!table) return cone_self(D, p);
+    const float4 c = *table;
+    return ConeSelf{c.x, c.y, c.z, c.w};
 }
 
 // The reference's crystal test, exactly (IEEE single, no contraction).
@@ -326,6 +333,18 @@ __device__ __forceinline__ bool plate_traversed(const Vec3& p, const Vec3& q, fl
     return !(plate_chord_exact(p, q, b) < 0.1f);
 }
 
+// plate_traversed for every ray of the bundle A -> B at once: its lateral window
+// between the plate's depth planes stays a further margin inside.
+__device__ __forceinline__ bool plate_sure(const Bundle& b, const PlateBox& pb) {
+    if (!b.ordered || !(b.A.y2 < pb.y1 - kMargin) || !(b.B.y1 > pb.y2 + kMargin) || !(pb.y2 - pb.y1 > 0.11f)) return false;
+    const float l1 = (pb.y1 - b.A.y2) * b.inv2, l2 = (pb.y2 - b.A.y1) * b.inv1;
+    const float lo_x = pb.x1 + 2.0f * kMargin, hi_x = pb.x2 - 2.0f * kMargin;
+    const float lo_z = pb.z1 + 2.0f * kMargin, hi_z = pb.z2 - 2.0f * kMargin;
+    const float ax = b.B.x1 - b.A.x1, bx = b.B.x2 - b.A.x2, az = b.B.z1 - b.A.z1, bz = b.B.z2 - b.A.z2;
+    return fminf(fmaf(ax, l1, b.A.x1), fmaf(ax, l2, b.A.x1)) > lo_x && fmaxf(fmaf(bx, l1, b.A.x2), fmaf(bx, l2, b.A.x2)) < hi_x &&
+           fminf(fmaf(az, l1, b.A.z1), fmaf(az, l2, b.A.z1)) > lo_z && fmaxf(fmaf(bz, l1, b.A.z2), fmaf(bz, l2, b.A.z2)) < hi_z;
+}
+
 __device__ __noinline__ float self_path_exact(Vec3 ps, Vec3 qs, Box3 crystal, Box3 unit, float* absorb_len, float r) {
     float l1 = chord_to_end(ps.x, ps.y, ps.z, qs.x, qs.y, qs.z, crystal);
     float l2 = chord_to_end(ps.x, ps.y, ps.z, qs.x, qs.y, qs.z, unit);
@@ -339,7 +358,8 @@ __device__ __noinline__ float self_path_exact(Vec3 ps, Vec3 qs, Box3 crystal, Bo
 // Contribution of one ray once its attenuation outside the detecting crystal
 // is known: the path inside the detecting crystal, absorption and solid angle.
 __device__ __forceinline__ float ray_value(const Detecting& D, const Vec3& ps, float xDs, float yDs, float zDs,
-                                           float att, float r, float inv_r, float dxw, float dy, float dzw) {
+                                           float att, float r, float inv_r, const ChordRay& cr, float dxw, float dy,
+                                           float dzw) {
     // Path inside the detecting crystal before the sub-cell and the absorption
     // chord (PESysMatGen.cu:727-759), as values: for the line from ps through
     // the sub-cell centre qs (direction u), the sub-cell entry lies at
@@ -348,19 +368,25 @@ __device__ __forceinline__ float ray_value(const Detecting& D, const Vec3& ps, f
     // crystal face facing ps.  When ps is not clearly outside the crystal or
     // the ray is nearly parallel to its depth faces, the reference's own
     // functions are used.
+    // (An unrotated crystal's frame is the world's: the ray's own reciprocals serve.)
     const float vx = xDs - ps.x, vy = yDs - ps.y, vz = zDs - ps.z;
+    float ux = cr.ax, uz = cr.az;
+    const float uy = cr.ay;
+    if (D.rotated) {
+        ux = fabsf(chord_rcp(vx));
+        uz = fabsf(chord_rcp(vz));
+    }
     float self_len, absorb_len;
     const float hw = 0.5f * D.w, ht = 0.5f * D.t, hh = 0.5f * D.h;
     const bool outside = (fabsf(ps.x) > hw + kMargin) || (fabsf(ps.y) > ht + kMargin) || (fabsf(ps.z) > hh + kMargin);
     if (outside && fabsf(vy) > 0.01f) {
-        const float ax = fabsf(vx), ay = fabsf(vy), az = fabsf(vz);
-        // distances along the line, in units of |v| * (1 / |v_i|)
-        const float cell = fminf(fminf(D.hx * __fdividef(1.0f, ax), D.hy * __fdividef(1.0f, ay)),
-                                 D.hz * __fdividef(1.0f, az));
+        // distances along the line, in units of |v| * (1 / |v_i|); a component of 0
+        // (reciprocal infinite or NaN) never is the smallest
+        const float cell = fminf(fminf(D.hx * ux, D.hy * uy), D.hz * uz);
         const float gx = (vx > 0.0f) ? (xDs + hw) : (hw - xDs);
         const float gy = (vy > 0.0f) ? (yDs + ht) : (ht - yDs);
         const float gz = (vz > 0.0f) ? (zDs + hh) : (hh - zDs);
-        const float crys = fminf(fminf(gx * __fdividef(1.0f, ax), gy * __fdividef(1.0f, ay)), gz * __fdividef(1.0f, az));
+        const float crys = fminf(fminf(gx * ux, gy * uy), gz * uz);
         self_len = (crys - cell) * r;
         absorb_len = 2.0f * cell * r;
     } else {
@@ -409,7 +435,7 @@ __device__ __forceinline__ SubCell sub_cell(const Detecting& D, const PeSmem& S,
 // mode also the hit record.
 template <bool RECORD>
 __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry& G, const PeSmem& S,
-                                           const WarpLists& L, const unsigned* pass_c, const unsigned* pass_h,
+                                           const WarpLists& L, unsigned plates_sure, bool any_hole,
                                            const float4* csp, const Detecting& D, const Vec3& p,
                                            const Vec3& ps, const SubCell& cell, int* rec, int* status,
                                            unsigned long long* n_cry, unsigned long long* n_hole,
@@ -417,23 +443,16 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
     const float xDs = cell.xDs, yDs = cell.yDs, zDs = cell.zDs;
     const Vec3 q = cell.q;
 
-    RaySeg seg;
-    seg.p = p;
-    seg.q = q;
-    seg.ordered = p.y < q.y;
-    const float dy = q.y - p.y;
-    seg.inv_dy = __fdividef(1.0f, dy);
-
-    unsigned plate_miss = 0u;
-    for (int m = 0; m < G.n_plates; ++m)
-        if (!plate_traversed(p, q, seg.inv_dy, G.plate[m])) plate_miss |= 1u << m;
-    if (!RECORD && plate_miss) return 0.0f;   // exp(-(1e5 + ...)) == 0
-
-    const float dxw = q.x - p.x, dzw = q.z - p.z;
+    const float dxw = q.x - p.x, dy = q.y - p.y, dzw = q.z - p.z;
     const float dsq = fmaf(dy, dy, fmaf(dxw, dxw, dzw * dzw));
     const float inv_r = rsqrtf(dsq);
     const float r = dsq * inv_r;
-    const ChordRay cr = make_chord_ray(p.x, p.y, p.z, dxw, dy, dzw, r);
+    const ChordRay cr = make_chord_ray(p.x, p.y, p.z, dxw, dy, dzw, r, P.chord_delta);
+
+    unsigned plate_miss = 0u;
+    for (int m = 0; m < G.n_plates; ++m)
+        if (!((plates_sure >> m) & 1u) && !plate_traversed(p, q, cr.iy, G.plate[m])) plate_miss |= 1u << m;
+    if (!RECORD && plate_miss) return 0.0f;   // exp(-(1e5 + ...)) == 0
 
     int rec_h = 0, rec_c = 0;
     float att = 0.0f;
@@ -441,30 +460,33 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
     // (PESysMatGen.cu:661-685).
     for (int m = 0; m < G.n_plates; ++m) {
         float in_holes = 0.0f;
-        const int hb = L.plate_begin[m], he = L.plate_begin[m + 1];
+        const int hb = any_hole ? L.plate_begin[m] : 0, he = any_hole ? L.plate_begin[m + 1] : 0;
         for (int wd = hb >> 5; wd <= ((he - 1) >> 5) && he > hb; ++wd) {
-            unsigned bits = pass_h[wd];
+            unsigned bits = L.pass_h[wd];
             const int lo = hb - (wd << 5), hi = he - (wd << 5);
             if (lo > 0) bits &= ~0u << lo;
             if (hi < 32) bits &= (1u << hi) - 1u;
             while (bits) {
                 const int b = __ffs(bits) - 1;
                 bits &= bits - 1;
-                const int e = L.list_h[(wd << 5) + b], k = e & (kConeSure - 1);
+                const int e = L.list_h[(wd << 5) + b], k = e & kIndex;
                 const float4 ha = S.h_a[k], hbv = S.h_b[k];
-                if (dy > 0.0f && p.y < ha.y &&
-                    hole_missed(p.x, p.y, p.z, dxw, dzw, cr.iy, ha.x, ha.y, ha.z, ha.w, hbv.x, kMargin))
-                    continue;
-                if (n_hole) ++*n_hole;
-                const float len = hole_chord_exact(p, q, ha, hbv.x);
-                if (len == 0.0f) continue;
+                float len = 0.0f;
+                int f = -1;
+                if (dy > 0.0f && p.y < ha.y)
+                    f = hole_filter(p.x, p.y, p.z, dxw, dzw, cr.iy, r, ha.x, ha.y, ha.z, ha.w, hbv.x, P.chord_delta, &len);
+                if (n_hole && f) ++*n_hole;
+                if (f < 0) {
+                    len = hole_chord_exact(p, q, ha, hbv.x);
+                    f = len != 0.0f;
+                }
+                if (!f) continue;
                 if (!(e & kConeSure)) {
                     if (n_cone) ++*n_cone;
-                    const float4 c4 = *csp;
-                    const ConeSelf cs{c4.x, c4.y, c4.z, c4.w};
-                    int f = cone_filter(cs, p, ha.x, hbv.w, ha.w, hbv.z);
-                    if (f < 0) f = cone_hole_exact(cs, p, ha.x, hbv.w, ha.w, hbv.z) ? 1 : 0;
-                    if (!f) continue;
+                    const ConeSelf cs = cone_of(csp, D, p);
+                    int g = cone_filter(cs, p, ha.x, hbv.w, ha.w, hbv.z);
+                    if (g < 0) g = cone_hole_exact(cs, p, ha.x, hbv.w, ha.w, hbv.z) ? 1 : 0;
+                    if (!g) continue;
                 }
                 in_holes += len;
                 att += hbv.y * len;
@@ -476,29 +498,34 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             }
         }
         const PlateBox& pb = G.plate[m];
-        const float through = pb.thickness * r * seg.inv_dy;   // T / cos(theta)
+        const float through = pb.thickness * r * cr.iy;   // T / cos(theta)
         if ((through - in_holes) >= 0.00001f) att += pb.mu_total * (through - in_holes);
     }
     // Other crystals among the candidates, each in its own frame (:687-725).
     const int nwc = (L.n_c + 31) >> 5;
     for (int wd = 0; wd < nwc; ++wd) {
-        unsigned bits = pass_c[wd];
+        unsigned bits = L.pass_c[wd];
         while (bits) {
             const int b = __ffs(bits) - 1;
             bits &= bits - 1;
-            const int e = L.list_c[(wd << 5) + b], k = e & (kConeSure - 1);
+            const int e = L.list_c[(wd << 5) + b], k = e & kIndex;
             const float4 kp = S.c_pos[k], kh = S.c_half[k];
-            const float kc = S.c_lo[k].w, ks = S.c_hi[k].w;   // cos, sin of the crystal's rotation
-            float len = 0.0f;
+            float len = 0.0f, kc = 1.0f, ks = 0.0f;   // cos, sin of the crystal's rotation
             int f;
-            if (kc == 1.0f && ks == 0.0f) {
-                f = chord_filter(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, P.chord_delta, &len);
+            if (!(e & kRotated)) {
+                f = chord_quick(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, &len);
+                if (f < 0) f = chord_filter(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, P.chord_delta, &len);
             } else {
+                kc = S.c_lo[k].w;
+                ks = S.c_hi[k].w;
                 // the segment in the crystal's frame; its rotation rounds once more, hence twice the margin
                 const float px = p.x - kp.x, pz = p.z - kp.z;
                 const ChordRay kr = make_chord_ray(fmaf(px, kc, -pz * ks), p.y - kp.y, fmaf(px, ks, pz * kc),
-                                                   fmaf(dxw, kc, -dzw * ks), dy, fmaf(dxw, ks, dzw * kc), r);
-                f = kr.ok ? chord_filter(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, 2.0f * P.chord_delta, &len) : -1;
+                                                   fmaf(dxw, kc, -dzw * ks), dy, fmaf(dxw, ks, dzw * kc), r,
+                                                   2.0f * P.chord_delta);
+                f = kr.ok ? chord_quick(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, &len) : -1;
+                if (f < 0 && kr.ok)
+                    f = chord_filter(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, 2.0f * P.chord_delta, &len);
             }
             if (n_cry && f) ++*n_cry;
             if (f < 0 || !cr.ok) {
@@ -508,8 +535,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             if (!f) continue;
             if (!(e & kConeSure)) {
                 if (n_cone) ++*n_cone;
-                const float4 c4 = *csp;
-                const ConeSelf cs{c4.x, c4.y, c4.z, c4.w};
+                const ConeSelf cs = cone_of(csp, D, p);
                 int g = cone_filter(cs, p, kp.x, kp.y, kp.z, kh.w);
                 if (g < 0) g = cone_crystal_exact(cs, p, kp.x, kp.y, kp.z, 2.0f * kh.w) ? 1 : 0;
                 if (!g) continue;
@@ -529,7 +555,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
         if (plate_miss) return 0.0f;
     }
 
-    return ray_value(D, ps, xDs, yDs, zDs, att, r, inv_r, dxw, dy, dzw);
+    return ray_value(D, ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
 }
 
 // One ray with its candidates read straight from the geometry tables: every
@@ -547,16 +573,16 @@ __device__ __forceinline__ float trace_ray_global(const DevGeometry& G, const De
     seg.p = p;
     seg.q = q;
     seg.ordered = p.y < q.y;
-    const float dy = q.y - p.y;
-    seg.inv_dy = __fdividef(1.0f, dy);
+    const float dxw = q.x - p.x, dy = q.y - p.y, dzw = q.z - p.z;
+    const float dsq = fmaf(dy, dy, fmaf(dxw, dxw, dzw * dzw));
+    const float inv_r = rsqrtf(dsq);
+    const float r = dsq * inv_r;
+    const ChordRay cr = make_chord_ray(p.x, p.y, p.z, dxw, dy, dzw, r, 0.0f);
+    seg.inv_dy = cr.iy;
     unsigned plate_miss = 0u;
     for (int m = 0; m < G.n_plates; ++m)
         if (!plate_traversed(p, q, seg.inv_dy, G.plate[m])) plate_miss |= 1u << m;
     if (!RECORD && plate_miss) return 0.0f;
-    const float dxw = q.x - p.x, dzw = q.z - p.z;
-    const float dsq = fmaf(dy, dy, fmaf(dxw, dxw, dzw * dzw));
-    const float inv_r = rsqrtf(dsq);
-    const float r = dsq * inv_r;
     int rec_h = 0, rec_c = 0;
     float att = 0.0f;
     for (int m = 0; m < G.n_plates; ++m) {
@@ -614,14 +640,14 @@ __device__ __forceinline__ float trace_ray_global(const DevGeometry& G, const De
         rec[2 + kRecHoles] = rec_c < kRecCrystals ? rec_c : kRecCrystals;
         if (plate_miss) return 0.0f;
     }
-    return ray_value(D, ps, xDs, yDs, zDs, att, r, inv_r, dxw, dy, dzw);
+    return ray_value(D, ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
 }
 
 // The warp's sum over every ray of voxel (ix, iy, iz) for detecting crystal d
 // through trace_ray_global (same value on every lane); taken only for voxels
 // whose candidates overflow the lists.
 template <bool RECORD>
-__device__ __forceinline__ float slow_voxel(const PEParams& P, const DevGeometry& G, const PeSmem& S, const Detecting& D,
+__device__ __noinline__ float slow_voxel(const PEParams& P, const DevGeometry& G, const PeSmem& S, const Detecting& D,
                                          int d, int ix, int iy, int iz, int rec_slot, int lane) {
     float acc = 0.0f, comp = 0.0f;
     const int n = P.n_sv * P.n_sc;
@@ -810,12 +836,13 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
     const int d = d0 + warp;
     WarpLists& L = S.wl[warp];
     if (d < P.row1) {
-        Detecting D;
-        {
+        if (lane == 0) {
+            Detecting D;
             const float4 pos = G.c.pos[d], sz = G.c.size[d], rt = G.c.rot[d], ph = G.c.phys[d];
             D.cx = pos.x; D.cy = pos.y; D.cz = pos.z; D.mu_t = pos.w; D.pe_frac = ph.x / pos.w;
             D.w = sz.x; D.t = sz.y; D.h = sz.z; D.crit = sz.w;
             D.cm = rt.x; D.sm = rt.y; D.cp = rt.z; D.sp = rt.w;
+            D.rotated = D.cm != 1.0f || D.sm != 0.0f;
             D.world = S.d_box[warp];
             D.area_x = D.t * D.h / (float)P.dZ / (float)P.dY;
             D.area_z = D.w * D.t / (float)P.dX / (float)P.dY;
@@ -823,7 +850,10 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
             D.hx = 0.5f * D.w / (float)P.dX;
             D.hy = 0.5f * D.t / (float)P.dY;
             D.hz = 0.5f * D.h / (float)P.dZ;
+            L.det = D;
         }
+        __syncwarp();
+        const Detecting& D = L.det;
         const bool absorbing = D.mu_t > 0.01f;   // PESysMatGen.cu:504, :598
         // Candidates the whole brick can reach for this crystal (bundle from the
         // brick's sub-point box A): the per-voxel lists narrow from these when
@@ -858,31 +888,51 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
         // (P.pair, up to 8): a pass then traces one sub-cell column from all of
         // them, and the lanes of each voxel are summed apart.
         const int VP = RECORD ? 1 : P.pair;
+        if (lane < P.dX * P.dZ && lane < kColTable) {
+            const SubCell c = sub_cell(D, S, lane % P.dX, 0, lane / P.dX);
+            L.col[lane] = make_float4(c.xDs, c.zDs, c.q.x, c.q.z);
+        }
+        __syncwarp();
+        unsigned plates_sure = 0u;   // plates that every ray of the brick to this crystal traverses
+        {
+            const Bundle bb = make_bundle(A, D.world);
+            for (int m = 0; m < G.n_plates; ++m) plates_sure |= plate_sure(bb, G.plate[m]) ? 1u << m : 0u;
+        }
+        // depth range of the crystal's sub-cell centres
+        const float cell_y1 = D.cy + (-D.t / 2.0f + S.frac[1][0] * D.t);
+        const float cell_y2 = D.cy + (-D.t / 2.0f + S.frac[1][P.dY - 1] * D.t);
+        // Lanes per voxel of a group, when a column's rays fill the pass and each
+        // voxel's lanes are a run of a power of two.
+        const int run = P.n_sv * P.dY;
+        const int span = VP == 1 ? 32 : ((VP * run == 32 && (run & (run - 1)) == 0) ? run : 0);
+        const float inv_span = span ? 1.0f / (float)span : 0.0f;
         // Flagging the candidates that surely pass the cone test pays once a voxel's
         // lists serve four passes or more (one pass per list: 7 % slower with it).
         const bool flag_sure = P.pair == 1 && P.n_sv * P.n_sc >= 128;
         for (int vl = 0; vl < tv; vl += VP) {
-            // voxel u of the group is brick voxel vl + u
+            // voxel u of the group is brick voxel vl + u; lane u (and every eighth lane after it) holds it
             auto vox_of = [&](int u, int& x, int& y, int& z) {
                 const int b = vl + u;
-                x = ix0 + b % P.bx;
-                y = iy0 + (b / P.bx) % P.by;
-                z = iz0 + b / (P.bx * P.by);
+                const int zb = fast_div(b, P.bx * P.by, P.inv_bxy), rem = b - zb * P.bx * P.by;
+                const int yb = fast_div(rem, P.bx, P.inv_bx);
+                x = ix0 + rem - yb * P.bx;
+                y = iy0 + yb;
+                z = iz0 + zb;
             };
             int ix, iy, iz;
-            vox_of(0, ix, iy, iz);
-            unsigned valid = 0u;
-            int lox = 1 << 30, loy = 1 << 30, loz = 1 << 30, hix = -1, hiy = -1, hiz = -1;
-            for (int u = 0; u < VP; ++u) {
-                int x, y, z;
-                vox_of(u, x, y, z);
-                if (vl + u < tv && x < ix1 && y < iy1 && z < iz1) {
-                    valid |= 1u << u;
-                    lox = min(lox, x); loy = min(loy, y); loz = min(loz, z);
-                    hix = max(hix, x); hiy = max(hiy, y); hiz = max(hiz, z);
-                }
-            }
+            vox_of(VP == 1 ? 0 : (lane & 7), ix, iy, iz);
+            const bool in = (lane & 7) < VP && vl + (lane & 7) < tv && ix < ix1 && iy < iy1 && iz < iz1;
+            const unsigned valid = __ballot_sync(0xffffffffu, in) & 0xffu;
             if (!valid) continue;
+            int lox = ix, loy = iy, loz = iz, hix = ix, hiy = iy, hiz = iz;
+            if (VP > 1) {
+                lox = __reduce_min_sync(0xffffffffu, in ? ix : 1 << 30);
+                loy = __reduce_min_sync(0xffffffffu, in ? iy : 1 << 30);
+                loz = __reduce_min_sync(0xffffffffu, in ? iz : 1 << 30);
+                hix = __reduce_max_sync(0xffffffffu, in ? ix : -1);
+                hiy = __reduce_max_sync(0xffffffffu, in ? iy : -1);
+                hiz = __reduce_max_sync(0xffffffffu, in ? iz : -1);
+            }
             int rec_slot = -1;
             if (RECORD) {
                 const long long vox = ((long long)iz * P.ny + iy) * P.nx + ix;
@@ -891,7 +941,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                 if (rec_slot < 0) continue;
             }
             float acc = 0.0f, comp = 0.0f;
-            int lane_vox = 0;
+            int lane_vox = VP == 1 ? 0 : fast_div(lane, span ? span : 32, span ? inv_span : 0.03125f);
             if (absorbing) {
                 // Voxel-level candidate lists: staged crystals/holes the bundle from
                 // the sub-points of the group's voxels (the box of their voxel
@@ -913,8 +963,10 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                             k = brick ? (int)L.blist_c[i] : i;
                             pass = (brick || S.c_id[k] != d) && bundle_hit(bv, box_of(S.c_lo[k], S.c_hi[k]));
                             const float4 kp = S.c_pos[k];
-                            if (pass && flag_sure && cone_sure(mid, rho, kp.x, kp.y, kp.z, S.c_half[k].w, D.cx, D.cy, D.cz, 0.5f * D.crit))
-                                k |= kConeSure;
+                            const bool sure = pass && flag_sure && cone_sure(mid, rho, kp.x, kp.y, kp.z, S.c_half[k].w,
+                                                                             D.cx, D.cy, D.cz, 0.5f * D.crit);
+                            if (S.c_lo[k].w != 1.0f || S.c_hi[k].w != 0.0f) k |= kRotated;
+                            if (sure) k |= kConeSure;
                         }
                         cnt = warp_append(pass, k, L.list_c, cnt, kListC, lane);
                     }
@@ -943,7 +995,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                         int below = 0;
                         for (int i0 = 0; i0 < cnth; i0 += 32) {
                             const int i = i0 + lane;
-                            below += __popc(__ballot_sync(0xffffffffu, i < cnth && S.h_id[L.list_h[i] & (kConeSure - 1)] < first));
+                            below += __popc(__ballot_sync(0xffffffffu, i < cnth && S.h_id[L.list_h[i] & kIndex] < first));
                         }
                         if (lane == 0) L.plate_begin[m] = below;
                     }
@@ -968,135 +1020,157 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                 }
                 const int lc = L.n_c, lh = L.n_h;
                 const int nwc = (lc + 31) >> 5, nwh = (lh + 31) >> 5;
-                // points of the group: the sub-points of voxel 0, then of voxel 1, ...
+                // Points of the voxels: the sub-points of voxel 0, then of voxel 1, ...
+                // They are traced in groups of P.group (and one shorter group).  The
+                // rays of a group, ordered (sub-cell column, point, depth sub-cell), are
+                // dealt 32 to a warp pass: a pass traces the depth cells of one column
+                // (or a few) from neighbouring points, rays that run almost together
+                // through the plates and the crystals in front, so the lanes meet the
+                // same candidates.  Every full group deals the same sub-cells to the
+                // same passes, so a pass's sub-cells and candidates serve all of them.
                 const int n_pts = VP * P.n_sv;
-                for (int s0 = 0; s0 < n_pts; s0 += P.group) {
-                    const int gn = min(P.group, n_pts - s0);
-                    // The cone (ConeSelf) of each sub-point of the group, for the
-                    // cone tests trace_ray takes on the candidates a ray crosses.
-                    if (lane < gn) {
-                        const int u = (VP == 1) ? 0 : (s0 + lane) / P.n_sv;
-                        int x = ix, y = iy, z = iz;
-                        if (u > 0) vox_of(u, x, y, z);
-                        const Vec3 p = subpoint_of(P, x, y, z, s0 + lane - u * P.n_sv);
+                if (VP > 1) {   // one group: its points once for all passes
+                    if (lane < n_pts) {
+                        const int u = fast_div(lane, P.n_sv, P.inv_n_sv);
+                        int x, y, z;
+                        vox_of(u, x, y, z);
+                        const Vec3 p = subpoint_of(P, x, y, z, lane - u * P.n_sv);
                         const ConeSelf cs = cone_self(D, p);
                         L.cs[lane] = make_float4(cs.ux, cs.uy, cs.uz, cs.crit_self);
-                        L.pt[lane] = make_float4(p.x, p.y, p.z, 0.0f);
-                        L.pself[lane] = make_float4((p.x - D.cx) * D.cm - (p.z - D.cz) * D.sm, p.y - D.cy,
-                                                    (p.x - D.cx) * D.sm + (p.z - D.cz) * D.cm, 0.0f);
+                        L.pt[lane] = make_float4(p.x, p.y, p.z, __int_as_float(u));
                     }
                     __syncwarp();
-                    // Rays of the group, ordered (sub-cell column, sub-point, depth
-                    // sub-cell) and dealt 32 to a warp pass: a pass traces the depth
-                    // cells of one column (or a few) from neighbouring sub-points,
-                    // rays that run almost together through the plates and the
-                    // crystals in front, so the lanes meet the same candidates.
+                }
+                for (int g0 = 0; g0 < n_pts;) {
+                    const int gn = min(P.group, n_pts - g0);
+                    const int g1 = gn == P.group ? n_pts - n_pts % P.group : n_pts;
                     const int cb = gn * P.dY;                  // rays per sub-cell column
-                    const float inv_cb = 1.0f / (float)cb;
+                    const float inv_cb = __fdividef(1.0f, (float)cb);
                     const int nr = gn * P.n_sc;
-                    // Full groups of one voxel deal the same sub-cells to the same
-                    // passes, so the first group's pass masks serve the others.
-                    const bool keep = VP == 1 && gn == P.group && nr <= 32 * kPassSlots;
                     for (int q0 = 0; q0 < nr; q0 += 32) {
-                        const int slot = keep ? (q0 >> 5) : 0;
                         const int e = q0 + lane;
-                        bool active = e < nr;
-                        int j = 0, sx = 0, sy = 0, sz = 0, u = 0;
-                        if (active) {
+                        const bool has = e < nr;
+                        bool active = has;
+                        int j = 0, sx = 0, sy = 0, sz = 0;
+                        if (has) {
                             const int col = fast_div(e, cb, inv_cb);
                             const int r = e - col * cb;
                             j = fast_div(r, P.dY, P.inv_dY);
                             sy = r - j * P.dY;
                             sz = fast_div(col, P.dX, P.inv_dX);
                             sx = col - sz * P.dX;
-                            if (VP > 1) {
-                                u = (s0 + j) / P.n_sv;
-                                active = (valid >> u) & 1u;
-                                lane_vox = u;
-                            }
                         }
-                        const SubCell cell = sub_cell(D, S, sx, sy, sz);
+                        SubCell cell;
+                        if (P.dX * P.dZ <= kColTable) {
+                            const float4 cc = L.col[sz * P.dX + sx];
+                            cell.xDs = cc.x;
+                            cell.zDs = cc.y;
+                            cell.yDs = -D.t / 2.0f + S.frac[1][sy] * D.t;
+                            cell.q = Vec3{cc.z, D.cy + cell.yDs, cc.w};
+                        } else {
+                            cell = sub_cell(D, S, sx, sy, sz);
+                        }
+                        bool any_hole = lh > 0;
+                        __syncwarp();
                         if (nr <= 32) {
                             // One pass holds every ray of the group: its bundle is the
                             // voxel's own, which the list was built from.
                             if (lane < nwc) {
                                 const int n_in = lc - (lane << 5);
-                                L.pass_c[slot][lane] = n_in >= 32 ? 0xffffffffu : ((1u << n_in) - 1u);
+                                L.pass_c[lane] = n_in >= 32 ? 0xffffffffu : ((1u << n_in) - 1u);
                             }
                             if (lane < nwh) {
                                 const int n_in = lh - (lane << 5);
-                                L.pass_h[slot][lane] = n_in >= 32 ? 0xffffffffu : ((1u << n_in) - 1u);
+                                L.pass_h[lane] = n_in >= 32 ? 0xffffffffu : ((1u << n_in) - 1u);
                             }
-                        } else if (!(keep && s0 > 0)) {
-                            // The pass's bundle: from the voxel's sub-point box to the
-                            // box of its rays' sub-cell centres.
-                            float bx1 = active ? cell.q.x : 3.0e38f, bx2 = active ? cell.q.x : -3.0e38f;
-                            float by1 = active ? cell.q.y : 3.0e38f, by2 = active ? cell.q.y : -3.0e38f;
-                            float bz1 = active ? cell.q.z : 3.0e38f, bz2 = active ? cell.q.z : -3.0e38f;
-                            for (int o = 16; o > 0; o >>= 1) {
-                                bx1 = fminf(bx1, __shfl_xor_sync(0xffffffffu, bx1, o));
-                                bx2 = fmaxf(bx2, __shfl_xor_sync(0xffffffffu, bx2, o));
-                                by1 = fminf(by1, __shfl_xor_sync(0xffffffffu, by1, o));
-                                by2 = fmaxf(by2, __shfl_xor_sync(0xffffffffu, by2, o));
-                                bz1 = fminf(bz1, __shfl_xor_sync(0xffffffffu, bz1, o));
-                                bz2 = fmaxf(bz2, __shfl_xor_sync(0xffffffffu, bz2, o));
+                        } else {
+                            // The pass's bundle: from the voxels' sub-point box to the box
+                            // of its rays' sub-cell centres (whole columns in depth).
+                            Box3 qb{cell.q.x, cell_y1, cell.q.z, cell.q.x, cell_y2, cell.q.z};
+                            if (cb % 32 != 0) {
+                                if (!has) qb.x1 = qb.z1 = 3.0e38f, qb.x2 = qb.z2 = -3.0e38f;
+                                for (int o = 16; o > 0; o >>= 1) {
+                                    qb.x1 = fminf(qb.x1, __shfl_xor_sync(0xffffffffu, qb.x1, o));
+                                    qb.x2 = fmaxf(qb.x2, __shfl_xor_sync(0xffffffffu, qb.x2, o));
+                                    qb.z1 = fminf(qb.z1, __shfl_xor_sync(0xffffffffu, qb.z1, o));
+                                    qb.z2 = fmaxf(qb.z2, __shfl_xor_sync(0xffffffffu, qb.z2, o));
+                                }
                             }
-                            const Bundle bq = make_bundle(Avox, Box3{bx1, by1, bz1, bx2, by2, bz2});
+                            const Bundle bq = make_bundle(Avox, qb);
                             // Narrow the voxel's candidates to those the pass can reach; a
                             // candidate dropped here is one that no ray of the pass can
-                            // reach, i.e. one trace_ray would skip by its own window test.
+                            // reach, i.e. one whose chord is 0 for every ray of the pass.
                             for (int w = 0; w < nwc; ++w) {
                                 bool pass = false;
                                 if ((w << 5) + lane < lc) {
-                                    const int k = L.list_c[(w << 5) + lane] & (kConeSure - 1);
+                                    const int k = L.list_c[(w << 5) + lane] & kIndex;
                                     pass = bundle_hit(bq, box_of(S.c_lo[k], S.c_hi[k]));
                                 }
                                 const unsigned bal = __ballot_sync(0xffffffffu, pass);
-                                if (lane == 0) L.pass_c[slot][w] = bal;
+                                if (lane == 0) L.pass_c[w] = bal;
                             }
+                            any_hole = false;
                             for (int w = 0; w < nwh; ++w) {
                                 bool pass = false;
                                 if ((w << 5) + lane < lh) {
-                                    const int k = L.list_h[(w << 5) + lane] & (kConeSure - 1);
+                                    const int k = L.list_h[(w << 5) + lane] & kIndex;
                                     pass = bundle_hit(bq, hole_box(S.h_a[k], S.h_b[k]));
                                 }
                                 const unsigned bal = __ballot_sync(0xffffffffu, pass);
-                                if (lane == 0) L.pass_h[slot][w] = bal;
+                                any_hole |= bal != 0u;
+                                if (lane == 0) L.pass_h[w] = bal;
                             }
                         }
                         __syncwarp();
-                        if (active) {
-                            const float4 p4 = L.pt[j], ps4 = L.pself[j];
-                            const Vec3 p{p4.x, p4.y, p4.z};
-                            const Vec3 ps{ps4.x, ps4.y, ps4.z};
-                            int* rec = nullptr;
-                            if (RECORD) {
-                                const int c = (sz * P.dX + sx) * P.dY + sy;   // the oracle's sub-cell order
-                                rec = P.rec_out + ((long long)rec_slot * P.n_sv * P.n_sc + (long long)(s0 + j) * P.n_sc + c) *
-                                                      kRecWords;
+                        for (int s0 = g0; s0 < g1; s0 += gn) {
+                            Vec3 p;
+                            const float4* csp = nullptr;
+                            if (VP > 1) {
+                                const float4 p4 = L.pt[j];
+                                p = Vec3{p4.x, p4.y, p4.z};
+                                csp = &L.cs[j];
+                                if (has) lane_vox = __float_as_int(p4.w);
+                                active = has && ((valid >> lane_vox) & 1u);
                             }
-                            const float v = trace_ray<RECORD>(P, G, S, L, L.pass_c[slot], L.pass_h[slot], &L.cs[j], D,
-                                                              p, ps, cell, rec, P.status,
-                                                              pc_cry, pc_hole, pc_cone);
-                            if (P.counters) ++cnt_rays;
-                            // Kahan summation of the lane's rays.
-                            const float y = v - comp;
-                            const float t = acc + y;
-                            comp = (t - acc) - y;
-                            acc = t;
+                            if (active) {
+                                if (VP == 1) p = subpoint_of(P, ix, iy, iz, s0 + j);
+                                // ... in the detecting crystal's frame
+                                Vec3 ps{p.x - D.cx, p.y - D.cy, p.z - D.cz};
+                                if (D.rotated) ps = Vec3{ps.x * D.cm - ps.z * D.sm, ps.y, ps.x * D.sm + ps.z * D.cm};
+                                int* rec = nullptr;
+                                if (RECORD) {
+                                    const int c = (sz * P.dX + sx) * P.dY + sy;   // the oracle's sub-cell order
+                                    rec = P.rec_out + ((long long)rec_slot * P.n_sv * P.n_sc + (long long)(s0 + j) * P.n_sc + c) *
+                                                          kRecWords;
+                                }
+                                const float v = trace_ray<RECORD>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
+                                                                  P.status, pc_cry, pc_hole, pc_cone);
+                                if (P.counters) ++cnt_rays;
+                                // Kahan summation of the lane's rays.
+                                const float y2 = v - comp;
+                                const float t = acc + y2;
+                                comp = (t - acc) - y2;
+                                acc = t;
+                            }
                         }
-                        __syncwarp();
                     }
-                    __syncwarp();
+                    g0 = g1;
                 }
             }
-            const float v = acc - comp;
-            for (int u = 0; u < VP; ++u) {
-                // a lane's rays all belong to one voxel of the group (pe_plan
-                // picks VP so that the lane-to-point map is the same every pass)
-                float w = lane_vox == u ? v : 0.0f;
-                for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-                if (lane == 0 && ((valid >> u) & 1u)) S.out[warp][vl + u] = w * P.inv_sv;
+            float v = acc - comp;
+            if (span) {
+                // the voxels' lanes are runs of `span` (a power of two): one butterfly within each
+                for (int o = span >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if ((lane & (span - 1)) == 0 && lane < span * VP && ((valid >> lane_vox) & 1u))
+                    S.out[warp][vl + lane_vox] = v * P.inv_sv;
+            } else {
+                for (int u = 0; u < VP; ++u) {
+                    // a lane's rays all belong to one voxel of the group (pe_plan
+                    // picks VP so that the lane-to-point map is the same every pass)
+                    float w = lane_vox == u ? v : 0.0f;
+                    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+                    if (lane == 0 && ((valid >> u) & 1u)) S.out[warp][vl + u] = w * P.inv_sv;
+                }
             }
         }
         if (P.counters) {
@@ -1131,7 +1205,8 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
 }
 
 template <bool RECORD>
-__global__ void __launch_bounds__(kPeThreads, 2) pe_trace_kernel(PEParams P, DevGeometry G) {
+__global__ void __launch_bounds__(kPeThreads, 2) pe_trace_kernel(const __grid_constant__ PEParams P,
+                                                                const __grid_constant__ DevGeometry G) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PeSmem& S = *reinterpret_cast<PeSmem*>(smem_raw);
     const long long tile = P.tile_list ? P.tile_list[blockIdx.x] : (long long)blockIdx.x;

@@ -181,6 +181,7 @@ int derive_into_stage(const float* col, size_t n_col, const float* det, size_t n
         float* hi = c_hi + 4 * (size_t)d;
         lo[0] = D[1] - ex; lo[1] = cy - t / 2.0f; lo[2] = D[3] - ez; lo[3] = 0.0f;
         hi[0] = D[1] + ex; hi[1] = cy + t / 2.0f; hi[2] = D[3] + ez; hi[3] = 0.0f;
+        add_crystal_box(&g, d, lo, hi);
     }
     return SM_OK;
 }
@@ -260,7 +261,9 @@ extern "C" int sm_pe_compute_static(const float* collimator, size_t n_collimator
 
     cudaStream_t stream = (cudaStream_t)stream_ptr;
     PEParams P;
-    pe_plan(g, opt->sv, opt->sc, opt->tile_voxels, opt->group, rotation, row0, row1, g.nz, z0, nz, &P);
+    int sms = 148;
+    SM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    pe_plan(g, opt->sv, opt->sc, opt->tile_voxels, opt->group, rotation, row0, row1, g.nz, z0, nz, pe_slots(sms), &P);
     // The array keeps the previous call's contents: the status word must
     // start at zero, and the geometry region is overwritten in full.
     SM_CUDA(cudaMemsetAsync(base, 0, kStatusBytes, stream));

@@ -222,7 +222,9 @@ struct ChordRay {
     float px, py, pz;
     float ix, iy, iz, ax, ay, az;
     float len;
-    bool ok;      // no axis is near the reference's degenerate extent (0.001)
+    float margin;   // largest of delta |1/d_i|
+    float eps;      // the reference's 0.001 in units of the segment
+    bool ok;        // no axis is near the reference's degenerate extent (0.001)
 };
 
 // 1 / d to about one unit in the last place.
@@ -235,12 +237,15 @@ SM_HD float chord_rcp(float d) {
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
 
-SM_HD ChordRay make_chord_ray(float px, float py, float pz, float dx, float dy, float dz, float len) {
+SM_HD ChordRay make_chord_ray(float px, float py, float pz, float dx, float dy, float dz, float len,
+                             float delta) {
     ChordRay c;
     c.px = px; c.py = py; c.pz = pz;
     c.ix = chord_rcp(dx); c.iy = chord_rcp(dy); c.iz = chord_rcp(dz);
     c.ax = fabsf(c.ix); c.ay = fabsf(c.iy); c.az = fabsf(c.iz);
     c.len = len;
+    c.margin = delta * fmaxf(fmaxf(c.ax, c.ay), c.az);
+    c.eps = 0.001f * chord_rcp(len);
     c.ok = fminf(fminf(fabsf(dx), fabsf(dy)), fabsf(dz)) > 0.002f;
     return c;
 }
@@ -275,21 +280,60 @@ SM_HD int chord_filter(const ChordRay& r, float cx, float cy, float cz, float hx
     return -1;
 }
 
-// True when the segment a -> b (inv_dy = 1 / (b_y - a_y)) surely misses the hole
-// cylinder: between the depth planes y1, y2 its lateral distance to the axis stays
-// above R + margin.  Valid for segments that run towards larger y.
-SM_HD bool hole_missed(float px, float py, float pz, float dx, float dz, float inv_dy, float xc, float y1, float y2,
-                       float zc, float R, float margin) {
-    const float l1 = (y1 - py) * inv_dy, l2 = (y2 - py) * inv_dy;
-    const float wx = xc - fmaf(dx, l1, px), wz = zc - fmaf(dz, l1, pz);
-    const float ex = dx * (l2 - l1), ez = dz * (l2 - l1);
+// The same call with one margin for all axes (the largest of delta |1/d_i|): a
+// third of the work, unclear more often for rays nearly parallel to a face.
+SM_HD int chord_quick(const ChordRay& r, float cx, float cy, float cz, float hx, float hy, float hz, float* chord) {
+    const float tx = (cx - r.px) * r.ix, ty = (cy - r.py) * r.iy, tz = (cz - r.pz) * r.iz;
+    const float lo = fmaxf(fmaxf(fmaf(-hx, r.ax, tx), fmaf(-hy, r.ay, ty)), fmaf(-hz, r.az, tz));
+    const float hi = fminf(fminf(fmaf(hx, r.ax, tx), fmaf(hy, r.ay, ty)), fmaf(hz, r.az, tz));
+    const float w = hi - lo, m = r.margin;
+    *chord = w * r.len;
+    if (w < r.eps - 2.0f * m || hi > 1.0f + m || lo < r.eps - m) return 0;
+    if (w > r.eps + 2.0f * m && hi < 1.0f - m && lo > r.eps + m) return 1;
+    return -1;
+}
+
+// chord_hole of a hole cylinder, when the answer is clear, for a segment that
+// runs towards larger y and starts before the hole: 1 (the chord), 0 (none) or -1
+// (chord_hole decides).  Between the depth planes y1 and y2 the segment moves
+// laterally from w (relative to the axis) by e; it crosses the wall where
+// |w + s e| = R.  Clear calls stay `margin` away from the wall at both planes (the
+// reference's points there round by a few units of 2^-24 of the coordinates), keep
+// to discriminants above twice the reference's floor and above 5 % of their
+// largest term (below, the reference-order form takes its value in double), and
+// start and end clear of the reference's end-point tests.
+SM_HD int hole_filter(float px, float py, float pz, float dx, float dz, float inv_dy, float len, float xc, float y1,
+                      float y2, float zc, float R, float margin, float* chord) {
+    const float l1 = (y1 - py) * inv_dy, l2 = (y2 - py) * inv_dy, dl = l2 - l1;
+    const float wx = fmaf(dx, l1, px) - xc, wz = fmaf(dz, l1, pz) - zc;
+    const float ex = dx * dl, ez = dz * dl;
     const float ee = fmaf(ex, ex, ez * ez), we = fmaf(wx, ex, wz * ez);
-    const float reach = R + margin, r2 = reach * reach;
     const float ww = fmaf(wx, wx, wz * wz);
-    if (we <= 0.0f) return ww > r2;                                   // nearest at the y1 plane
-    if (we >= ee) return ww - 2.0f * we + ee > r2;                    // ... at the y2 plane
+    const float far2 = (R + margin) * (R + margin), near2 = (R - margin) * (R - margin);
     const float cr = fmaf(wx, ez, -wz * ex);
-    return cr * cr > r2 * ee;
+    const bool between = we < 0.0f && we > -ee;         // the nearest point lies between the planes
+    const float vx = wx + ex, vz = wz + ez;
+    const float vv = fmaf(vx, vx, vz * vz);             // |w|^2 at the y2 plane
+    if (between ? cr * cr > far2 * ee : fminf(ww, vv) > far2) return 0;
+    if (!(R > margin) || !(l1 * len > 0.001f && l2 < 0.9999f) || (y2 - y1) < 0.01f) return -1;
+    const bool in_a = ww < near2, in_b = vv < near2;
+    if (!(in_a || ww > far2) || !(in_b || vv > far2)) return -1;
+    const float t = dl * len;
+    if (in_a && in_b) {
+        *chord = t;
+        return 1;
+    }
+    const float r2 = R * R, disc = fmaf(-cr, cr, ee * r2);
+    if (!(disc > 0.05f * ee * r2) || !(disc > 2e-5f * t * t)) return -1;
+    const float root = sqrtf(disc);
+    float s;
+    if (in_a) s = we > 0.0f ? (r2 - ww) / (root + we) : (root - we) / ee;
+    else if (in_b) {
+        const float ve = we + ee;                       // v . e
+        s = ve < 0.0f ? (r2 - vv) / (root - ve) : (root + ve) / ee;
+    } else s = 2.0f * root / ee;
+    *chord = s * t;
+    return 1;
 }
 
 // Conservative culling: can any segment from a point of box A to a point of

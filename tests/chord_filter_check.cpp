@@ -1,6 +1,7 @@
-// Compares the tracer's chord_filter and hole_missed with the reference-order
+// Compares the tracer's chord_quick, chord_filter and hole_filter with the reference-order
 // chord_through and chord_hole on the host: chord_filter_check SEED COUNT RANGE.
-// Prints "<wrong calls> <clear hits> <clear misses> <unclear> <largest value error>".
+// Prints "<wrong calls> <clear hits> <clear misses> <unclear> <largest value error>
+// <clear holes> <of them crossed> <unclear holes>".
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -18,7 +19,7 @@ int main(int argc, char** argv) {
     auto U = [&](float a, float b) { return std::uniform_real_distribution<float>(a, b)(gen); };
     auto side = [&](float h) { return U(0, 1) < 0.5f ? -h : h; };
     const float lat = 0.35f * range;   // image and detector half width; depth up to half the range
-    long wrong = 0, hits = 0, misses = 0, unclear = 0;
+    long wrong = 0, hits = 0, misses = 0, unclear = 0, hole_clear = 0, hole_hits = 0, hole_unclear = 0;
     double worst = 0.0;
     for (long i = 0; i < n; ++i) {
         const float hx = U(0.3f, 2), hy = U(0.3f, 4), hz = U(0.3f, 2), near = 3 * delta;
@@ -47,21 +48,24 @@ int main(int argc, char** argv) {
             pz = kz + U(-1, 1) * hz;
         }
         const float dx = qx - px, dy = qy - py, dz = qz - pz, len = std::sqrt(dx * dx + dy * dy + dz * dz);
-        const ChordRay r = make_chord_ray(px, py, pz, dx, dy, dz, len);
+        const ChordRay r = make_chord_ray(px, py, pz, dx, dy, dz, len, delta);
         const Box3 box{-hx, -hy, -hz, hx, hy, hz};
-        float chord = 0, ref;
-        int f;
+        float chord = 0, quick = 0, ref;
+        int f, fq;
         if (i % 3) {
             f = r.ok ? chord_filter(r, kx, ky, kz, hx, hy, hz, delta, &chord) : -1;
+            fq = r.ok ? chord_quick(r, kx, ky, kz, hx, hy, hz, &quick) : -1;
             ref = chord_through(px - kx, py - ky, pz - kz, qx - kx, qy - ky, qz - kz, box);
         } else {
             const float a = U(-0.5f, 0.5f), c = std::cos(a), s = std::sin(a), ax = px - kx, az = pz - kz;
             const ChordRay k = make_chord_ray(fmaf(ax, c, -az * s), py - ky, fmaf(ax, s, az * c), fmaf(dx, c, -dz * s), dy,
-                                              fmaf(dx, s, dz * c), len);
+                                              fmaf(dx, s, dz * c), len, 2 * delta);
             f = k.ok ? chord_filter(k, 0, 0, 0, hx, hy, hz, 2 * delta, &chord) : -1;
+            fq = k.ok ? chord_quick(k, 0, 0, 0, hx, hy, hz, &quick) : -1;
             ref = chord_through(ax * c - az * s, py - ky, ax * s + az * c, (qx - kx) * c - (qz - kz) * s, qy - ky,
                                 (qx - kx) * s + (qz - kz) * c, box);
         }
+        if (fq >= 0) wrong += (fq != 0) != (ref != 0) || (f >= 0 && f != fq) || (fq == 1 && f == 1 && quick != chord);
         if (f < 0) ++unclear;
         else if (f == 0) { ++misses; wrong += ref != 0; }
         else {
@@ -69,12 +73,31 @@ int main(int argc, char** argv) {
             wrong += ref == 0;
             worst = std::fmax(worst, std::fabs((double)chord - ref) / (delta * len * std::fmax(r.ax, std::fmax(r.ay, r.az))));
         }
-        // a hole of radius hx between ky - hy and ky + hy
-        if (py < ky - hy && dy > 0 &&
-            hole_missed(px, py, pz, dx, dz, r.iy, kx, ky - hy, ky + hy, kz, hx, 0.01f) &&
-            chord_hole(px, py, pz, qx, qy, qz, kx, ky - hy, ky + hy, kz, hx) != 0)
-            ++wrong;
+        // a hole of radius hx between ky - hy and ky + hy; every other one has its wall near the ray
+        if (py < ky - hy && dy > 0) {
+            float hxc = kx, hzc = kz;
+            if (i % 5 < 3) {
+                const float a = U(0, 6.2831853f), g = hx + U(-near, near), m = (ky + U(-hy, hy) - py) / dy;
+                const float m1 = i % 5 == 0 ? (ky - hy - py) / dy : m;
+                hxc = px + dx * m1 + g * std::cos(a);
+                hzc = pz + dz * m1 + g * std::sin(a);
+            }
+            float hc = 0;
+            const int hf = hole_filter(px, py, pz, dx, dz, r.iy, len, hxc, ky - hy, ky + hy, hzc, hx, delta, &hc);
+            const float hr = chord_hole(px, py, pz, qx, qy, qz, hxc, ky - hy, ky + hy, hzc, hx);
+            if (hf < 0) ++hole_unclear;
+            else {
+                ++hole_clear;
+                hole_hits += hf;
+                wrong += (hf != 0) != (hr != 0);
+                // the wall's crossing moves by the margin times the ray's slope to it, at most
+                // 1 / sqrt(0.05) times the slope to the axis for the discriminants kept
+                const float lat2 = dx * dx + dz * dz;
+                if (hf && hr != 0)
+                    worst = std::fmax(worst, std::fabs((double)hc - hr) / (10.0 * delta * len * std::fmax(std::fabs(r.iy), 1 / std::sqrt(lat2))));
+            }
+        }
     }
-    std::printf("%ld %ld %ld %ld %.3g\n", wrong, hits, misses, unclear, worst);
+    std::printf("%ld %ld %ld %ld %.3g %ld %ld %ld\n", wrong, hits, misses, unclear, worst, hole_clear, hole_hits, hole_unclear);
     return 0;
 }

@@ -1,4 +1,4 @@
-"""The tracer's division-free chord filter against the reference-order chord, on
+"""The tracer's chord filters (boxes, holes) against the reference-order chords, on
 the host: the same header (csrc/tracer.cuh) the kernels include.  The filter may
 call a chord unclear, never wrong; a clear chord lies within the filter's own
 margin of the exact one (both ends of the chord move by less than the margin
@@ -28,3 +28,4 @@ def test_clear_calls_are_the_exact_ones(check, coordinate_range):
     assert hits > 100000 and misses > 100000
     assert unclear < 0.35 * (hits + misses)      # every second ray aims at an edge
     assert float(out[4]) <= 2.0
+    assert int(out[6]) > 50000                    # three holes in five have their wall near the ray
