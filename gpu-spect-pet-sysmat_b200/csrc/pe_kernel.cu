@@ -474,7 +474,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
                 float len = 0.0f;
                 int f = -1;
                 if (dy > 0.0f && p.y < ha.y)
-                    f = hole_filter(p.x, p.y, p.z, dxw, dzw, cr.iy, r, ha.x, ha.y, ha.z, ha.w, hbv.x, P.chord_delta, &len);
+                    f = hole_filter(p.x, p.y, p.z, dxw, dy, dzw, cr.iy, r, ha.x, ha.y, ha.z, ha.w, hbv.x, P.chord_delta, &len);
                 if (n_hole && f) ++*n_hole;
                 if (f < 0) {
                     len = hole_chord_exact(p, q, ha, hbv.x);
@@ -498,7 +498,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             }
         }
         const PlateBox& pb = G.plate[m];
-        const float through = pb.thickness * r * cr.iy;   // T / cos(theta)
+        const float through = pb.thickness * r * fast_rcp(dy);   // T / cos(theta)
         if ((through - in_holes) >= 0.00001f) att += pb.mu_total * (through - in_holes);
     }
     // Other crystals among the candidates, each in its own frame (:687-725).
@@ -578,7 +578,7 @@ __device__ __forceinline__ float trace_ray_global(const DevGeometry& G, const De
     const float inv_r = rsqrtf(dsq);
     const float r = dsq * inv_r;
     const ChordRay cr = make_chord_ray(p.x, p.y, p.z, dxw, dy, dzw, r, 0.0f);
-    seg.inv_dy = cr.iy;
+    seg.inv_dy = fast_rcp(dy);
     unsigned plate_miss = 0u;
     for (int m = 0; m < G.n_plates; ++m)
         if (!plate_traversed(p, q, seg.inv_dy, G.plate[m])) plate_miss |= 1u << m;

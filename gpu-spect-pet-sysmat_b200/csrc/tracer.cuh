@@ -227,13 +227,17 @@ struct ChordRay {
     bool ok;        // no axis is near the reference's degenerate extent (0.001)
 };
 
+SM_HD float fast_rcp(float d) {
+#ifdef __CUDA_ARCH__
+    return __fdividef(1.0f, d);
+#else
+    return 1.0f / d;
+#endif
+}
+
 // 1 / d to about one unit in the last place.
 SM_HD float chord_rcp(float d) {
-#ifdef __CUDA_ARCH__
-    const float r = __fdividef(1.0f, d);
-#else
-    const float r = 1.0f / d;
-#endif
+    const float r = fast_rcp(d);
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
 
@@ -293,46 +297,66 @@ SM_HD int chord_quick(const ChordRay& r, float cx, float cy, float cz, float hx,
     return -1;
 }
 
-// chord_hole of a hole cylinder, when the answer is clear, for a segment that
-// runs towards larger y and starts before the hole: 1 (the chord), 0 (none) or -1
+// a / b with rb ~ 1 / b, and sqrt(x), each with one residual correction (Markstein,
+// IBM J. Res. Dev. 34 (1990) 111): the correctly rounded result but for about one
+// operand in 2^20, without the range checks of the IEEE forms.  For values only.
+SM_HD float near_div(float a, float b, float rb) {
+    const float q = a * rb;
+    return fmaf(fmaf(-q, b, a), rb, q);
+}
+
+SM_HD float near_sqrt(float x) {
+#ifdef __CUDA_ARCH__
+    const float r = rsqrtf(x);
+#else
+    const float r = 1.0f / std::sqrt(x);
+#endif
+    const float s = x * r;
+    return fmaf(fmaf(-s, s, x), 0.5f * r, s);
+}
+
+// chord_hole of a hole cylinder for a segment that runs towards larger y and
+// starts before the hole, when the answer is clear: 1 (the chord), 0 (none) or -1
 // (chord_hole decides).  Between the depth planes y1 and y2 the segment moves
-// laterally from w (relative to the axis) by e; it crosses the wall where
-// |w + s e| = R.  Clear calls stay `margin` away from the wall at both planes (the
-// reference's points there round by a few units of 2^-24 of the coordinates), keep
-// to discriminants above twice the reference's floor and above 5 % of their
-// largest term (below, the reference-order form takes its value in double), and
-// start and end clear of the reference's end-point tests.
-SM_HD int hole_filter(float px, float py, float pz, float dx, float dz, float inv_dy, float len, float xc, float y1,
-                      float y2, float zc, float R, float margin, float* chord) {
+// laterally from w (relative to the axis) by e.  Clear calls stay `margin` away
+// from the wall at both planes (the reference's points there round by a few
+// units of 2^-24 of the coordinates), clear of its end-point tests, above twice
+// its floor of the discriminant, and where it takes its roots in single precision
+// and a miss is far from a tangent.  The chord is then chord_hole's, operation for
+// operation: through tungsten an entry follows it times 3.5 / mm, so another
+// form's rounding of 4e-6 mm would show as 1.4e-5 of the entry.
+SM_HD int hole_filter(float px, float py, float pz, float dx, float dy, float dz, float inv_dy, float len, float xc,
+                      float y1, float y2, float zc, float R, float margin, float* chord) {
     const float l1 = (y1 - py) * inv_dy, l2 = (y2 - py) * inv_dy, dl = l2 - l1;
-    const float wx = fmaf(dx, l1, px) - xc, wz = fmaf(dz, l1, pz) - zc;
+    const float wx = fmaf(dx, l1, px) - xc, wz = fmaf(dz, l1, pz) - zc;   // from the axis, at the y1 plane
     const float ex = dx * dl, ez = dz * dl;
-    const float ee = fmaf(ex, ex, ez * ez), we = fmaf(wx, ex, wz * ez);
-    const float ww = fmaf(wx, wx, wz * wz);
+    const float vx = wx + ex, vz = wz + ez;                               // ... at the y2 plane
+    const float ww = fmaf(wx, wx, wz * wz), vv = fmaf(vx, vx, vz * vz);
     const float far2 = (R + margin) * (R + margin), near2 = (R - margin) * (R - margin);
+    const float ee = fmaf(ex, ex, ez * ez), we = fmaf(wx, ex, wz * ez);
     const float cr = fmaf(wx, ez, -wz * ex);
-    const bool between = we < 0.0f && we > -ee;         // the nearest point lies between the planes
-    const float vx = wx + ex, vz = wz + ez;
-    const float vv = fmaf(vx, vx, vz * vz);             // |w|^2 at the y2 plane
+    const bool between = we < 0.0f && we > -ee;                           // the nearest point lies between the planes
     if (between ? cr * cr > far2 * ee : fminf(ww, vv) > far2) return 0;
-    if (!(R > margin) || !(l1 * len > 0.001f && l2 < 0.9999f) || (y2 - y1) < 0.01f) return -1;
     const bool in_a = ww < near2, in_b = vv < near2;
-    if (!(in_a || ww > far2) || !(in_b || vv > far2)) return -1;
-    const float t = dl * len;
+    if (!(in_a || ww > far2) || !(in_b || vv > far2) || !(R > margin) || !(l1 * len > 0.001f && l2 < 0.9999f) ||
+        !(y2 - y1 > 0.01f))
+        return -1;
+    const float t = near_sqrt(dx * dx + dy * dy + dz * dz), rt = chord_rcp(t);
+    const float ky = near_div(dy, t, rt), rk = chord_rcp(ky);
+    const float t_a = near_div(y1 - py, ky, rk), t_b = near_div(y2 - py, ky, rk);
     if (in_a && in_b) {
-        *chord = t;
+        *chord = fabsf(t_b - t_a);
         return 1;
     }
-    const float r2 = R * R, disc = fmaf(-cr, cr, ee * r2);
-    if (!(disc > 0.05f * ee * r2) || !(disc > 2e-5f * t * t)) return -1;
-    const float root = sqrtf(disc);
-    float s;
-    if (in_a) s = we > 0.0f ? (r2 - ww) / (root + we) : (root - we) / ee;
-    else if (in_b) {
-        const float ve = we + ee;                       // v . e
-        s = ve < 0.0f ? (r2 - vv) / (root - ve) : (root + ve) / ee;
-    } else s = 2.0f * root / ee;
-    *chord = s * t;
+    const float kx = near_div(dx, t, rt), kz = near_div(dz, t, rt);
+    const float qx = px - xc, qz = pz - zc;
+    const float kk = kx * kx + kz * kz;
+    const float cross = kx * qz - kz * qx;
+    const float full = kk * R * R, disc = full - cross * cross;
+    if (!(disc > 0.05f * full) || !(disc > 2e-5f)) return -1;
+    const float sq = near_sqrt(disc), rkk = chord_rcp(kk), b = -(kx * qx + kz * qz);
+    const float t1 = near_div(b - sq, kk, rkk), t2 = near_div(b + sq, kk, rkk);
+    *chord = in_a ? t2 - t_a : (in_b ? t_b - t1 : t2 - t1);
     return 1;
 }
 

@@ -1,7 +1,7 @@
 // Compares the tracer's chord_quick, chord_filter and hole_filter with the reference-order
 // chord_through and chord_hole on the host: chord_filter_check SEED COUNT RANGE.
 // Prints "<wrong calls> <clear hits> <clear misses> <unclear> <largest value error>
-// <clear holes> <of them crossed> <unclear holes>".
+// <holes called missed> <holes called crossed> <of them with another value>".
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -19,7 +19,7 @@ int main(int argc, char** argv) {
     auto U = [&](float a, float b) { return std::uniform_real_distribution<float>(a, b)(gen); };
     auto side = [&](float h) { return U(0, 1) < 0.5f ? -h : h; };
     const float lat = 0.35f * range;   // image and detector half width; depth up to half the range
-    long wrong = 0, hits = 0, misses = 0, unclear = 0, hole_clear = 0, hole_hits = 0, hole_unclear = 0;
+    long wrong = 0, hits = 0, misses = 0, unclear = 0, hole_misses = 0, hole_hits = 0, hole_other = 0;
     double worst = 0.0;
     for (long i = 0; i < n; ++i) {
         const float hx = U(0.3f, 2), hy = U(0.3f, 4), hz = U(0.3f, 2), near = 3 * delta;
@@ -83,21 +83,14 @@ int main(int argc, char** argv) {
                 hzc = pz + dz * m1 + g * std::sin(a);
             }
             float hc = 0;
-            const int hf = hole_filter(px, py, pz, dx, dz, r.iy, len, hxc, ky - hy, ky + hy, hzc, hx, delta, &hc);
+            const int hf = hole_filter(px, py, pz, dx, dy, dz, r.iy, len, hxc, ky - hy, ky + hy, hzc, hx, delta, &hc);
             const float hr = chord_hole(px, py, pz, qx, qy, qz, hxc, ky - hy, ky + hy, hzc, hx);
-            if (hf < 0) ++hole_unclear;
-            else {
-                ++hole_clear;
-                hole_hits += hf;
-                wrong += (hf != 0) != (hr != 0);
-                // the wall's crossing moves by the margin times the ray's slope to it, at most
-                // 1 / sqrt(0.05) times the slope to the axis for the discriminants kept
-                const float lat2 = dx * dx + dz * dz;
-                if (hf && hr != 0)
-                    worst = std::fmax(worst, std::fabs((double)hc - hr) / (10.0 * delta * len * std::fmax(std::fabs(r.iy), 1 / std::sqrt(lat2))));
-            }
+            hole_misses += hf == 0;
+            hole_hits += hf == 1;
+            hole_other += hf == 1 && hc != hr;
+            wrong += (hf == 0 && hr != 0) || (hf == 1 && (hr == 0 || std::fabs(hc - hr) > 2e-6f * len));
         }
     }
-    std::printf("%ld %ld %ld %ld %.3g %ld %ld %ld\n", wrong, hits, misses, unclear, worst, hole_clear, hole_hits, hole_unclear);
+    std::printf("%ld %ld %ld %ld %.3g %ld %ld %ld\n", wrong, hits, misses, unclear, worst, hole_misses, hole_hits, hole_other);
     return 0;
 }
