@@ -66,7 +66,7 @@ static_assert(kSupC <= kIndex && kSupH <= kIndex, "staged-set indices share 16 b
 
 // Per-crystal constants of the warp's detecting crystal.
 struct Detecting {
-    float cx, cy, cz, mu_t, pe_frac;   // pe_frac = mu_pe / mu_t
+    float cx, cy, cz, mu_t, mu_pe, inv_mu;   // inv_mu = 1 / mu_t
     float w, t, h, crit;
     float cm, sm, cp, sp;          // cos(-rot), sin(-rot), cos(rot), sin(rot)
     Box3 world;                    // inflated world AABB
@@ -357,7 +357,7 @@ __device__ __noinline__ float self_path_exact(Vec3 ps, Vec3 qs, Box3 crystal, Bo
 
 // Contribution of one ray once its attenuation outside the detecting crystal
 // is known: the path inside the detecting crystal, absorption and solid angle.
-__device__ __forceinline__ float ray_value(const Detecting& D, const Vec3& ps, float xDs, float yDs, float zDs,
+__device__ __forceinline__ float ray_value(const Detecting& D, bool own_frame, const Vec3& ps, float xDs, float yDs, float zDs,
                                            float att, float r, float inv_r, const ChordRay& cr, float dxw, float dy,
                                            float dzw) {
     // Path inside the detecting crystal before the sub-cell and the absorption
@@ -368,13 +368,14 @@ __device__ __forceinline__ float ray_value(const Detecting& D, const Vec3& ps, f
     // crystal face facing ps.  When ps is not clearly outside the crystal or
     // the ray is nearly parallel to its depth faces, the reference's own
     // functions are used.
-    // (An unrotated crystal's frame is the world's: the ray's own reciprocals serve.)
+    // (An unrotated crystal's frame is the world's: the ray's own reciprocals serve,
+    // unless own_frame asks for those of the frame.)
     const float vx = xDs - ps.x, vy = yDs - ps.y, vz = zDs - ps.z;
-    float ux = cr.ax, uz = cr.az;
-    const float uy = cr.ay;
-    if (D.rotated) {
-        ux = fabsf(chord_rcp(vx));
-        uz = fabsf(chord_rcp(vz));
+    float ux = cr.ax, uy = cr.ay, uz = cr.az;
+    if (own_frame) {
+        ux = fast_rcp(fabsf(vx));
+        uy = fast_rcp(fabsf(vy));
+        uz = fast_rcp(fabsf(vz));
     }
     float self_len, absorb_len;
     const float hw = 0.5f * D.w, ht = 0.5f * D.t, hh = 0.5f * D.h;
@@ -396,7 +397,7 @@ __device__ __forceinline__ float ray_value(const Detecting& D, const Vec3& ps, f
     }
     att = fmaf(self_len, D.mu_t, att);
     const float eff = __expf(-att);
-    const float absorb = (1.0f - __expf(-absorb_len * D.mu_t)) * D.pe_frac;
+    const float absorb = near_div((1.0f - __expf(-absorb_len * D.mu_t)) * D.mu_pe, D.mu_t, D.inv_mu);
     // Solid angle: the largest of the three projected sub-cell faces (:618-639),
     // A * |cos| / (4 pi d^2).
     const float k4 = 0.0795774715459476678f * inv_r * inv_r * inv_r;   // 1 / (4 pi d^3)
@@ -433,7 +434,7 @@ __device__ __forceinline__ SubCell sub_cell(const Detecting& D, const PeSmem& S,
 // either way, so the cone test (`csp`: the sub-point's ConeSelf) is taken only
 // for candidates with a nonzero chord.  Returns the contribution; in RECORD
 // mode also the hit record.
-template <bool RECORD>
+template <bool RECORD, bool FEW>
 __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry& G, const PeSmem& S,
                                            const WarpLists& L, unsigned plates_sure, bool any_hole,
                                            const float4* csp, const Detecting& D, const Vec3& p,
@@ -511,6 +512,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             const int e = L.list_c[(wd << 5) + b], k = e & kIndex;
             const float4 kp = S.c_pos[k], kh = S.c_half[k];
             float len = 0.0f, kc = 1.0f, ks = 0.0f;   // cos, sin of the crystal's rotation
+            float kix = 0.0f, kiz = 0.0f;             // 1 / extents in its frame
             int f;
             if (!(e & kRotated)) {
                 f = chord_quick(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, &len);
@@ -523,6 +525,8 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
                 const ChordRay kr = make_chord_ray(fmaf(px, kc, -pz * ks), p.y - kp.y, fmaf(px, ks, pz * kc),
                                                    fmaf(dxw, kc, -dzw * ks), dy, fmaf(dxw, ks, dzw * kc), r,
                                                    2.0f * P.chord_delta);
+                kix = kr.ix;
+                kiz = kr.iz;
                 f = kr.ok ? chord_quick(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, &len) : -1;
                 if (f < 0 && kr.ok)
                     f = chord_filter(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, 2.0f * P.chord_delta, &len);
@@ -533,6 +537,17 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
                 f = len != 0.0f;
             }
             if (!f) continue;
+            if (FEW && f > 0 && cr.ok) {
+                // Entries of few rays keep the exact form's rounding (their matrices feed the
+                // scatter pipeline, whose bf16 operands and error estimates magnify it); entries
+                // of many rays average the filter's, which is of the same size.
+                const float ax = p.x - kp.x, az = p.z - kp.z, bx = q.x - kp.x, bz = q.z - kp.z;
+                if (!(e & kRotated))
+                    len = chord_value(ax, p.y - kp.y, az, bx, q.y - kp.y, bz, kh.x, kh.y, kh.z, cr.ix, cr.iy, cr.iz, inv_r);
+                else
+                    len = chord_value(ax * kc - az * ks, p.y - kp.y, ax * ks + az * kc, bx * kc - bz * ks, q.y - kp.y,
+                                      bx * ks + bz * kc, kh.x, kh.y, kh.z, kix, cr.iy, kiz, inv_r);
+            }
             if (!(e & kConeSure)) {
                 if (n_cone) ++*n_cone;
                 const ConeSelf cs = cone_of(csp, D, p);
@@ -555,7 +570,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
         if (plate_miss) return 0.0f;
     }
 
-    return ray_value(D, ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
+    return ray_value(D, FEW || D.rotated, ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
 }
 
 // One ray with its candidates read straight from the geometry tables: every
@@ -640,7 +655,7 @@ __device__ __forceinline__ float trace_ray_global(const DevGeometry& G, const De
         rec[2 + kRecHoles] = rec_c < kRecCrystals ? rec_c : kRecCrystals;
         if (plate_miss) return 0.0f;
     }
-    return ray_value(D, ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
+    return ray_value(D, true, ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
 }
 
 // The warp's sum over every ray of voxel (ix, iy, iz) for detecting crystal d
@@ -689,7 +704,7 @@ __device__ __forceinline__ int warp_append(bool pass, int value, unsigned short*
 
 // One tile (8 crystals x one voxel brick) of geometry G.  Shared by the
 // one-launch-per-geometry kernel and the persistent batch kernel.
-template <bool RECORD>
+template <bool RECORD, bool FEW>
 __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G, PeSmem& S, long long tile) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -839,7 +854,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
         if (lane == 0) {
             Detecting D;
             const float4 pos = G.c.pos[d], sz = G.c.size[d], rt = G.c.rot[d], ph = G.c.phys[d];
-            D.cx = pos.x; D.cy = pos.y; D.cz = pos.z; D.mu_t = pos.w; D.pe_frac = ph.x / pos.w;
+            D.cx = pos.x; D.cy = pos.y; D.cz = pos.z; D.mu_t = pos.w; D.mu_pe = ph.x; D.inv_mu = 1.0f / pos.w;
             D.w = sz.x; D.t = sz.y; D.h = sz.z; D.crit = sz.w;
             D.cm = rt.x; D.sm = rt.y; D.cp = rt.z; D.sp = rt.w;
             D.rotated = D.cm != 1.0f || D.sm != 0.0f;
@@ -887,7 +902,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
         // Entries of few rays go VP neighbouring voxels of the brick to a group
         // (P.pair, up to 8): a pass then traces one sub-cell column from all of
         // them, and the lanes of each voxel are summed apart.
-        const int VP = RECORD ? 1 : P.pair;
+        const int VP = FEW ? P.pair : 1;
         if (lane < P.dX * P.dZ && lane < kColTable) {
             const SubCell c = sub_cell(D, S, lane % P.dX, 0, lane / P.dX);
             L.col[lane] = make_float4(c.xDs, c.zDs, c.q.x, c.q.z);
@@ -908,7 +923,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
         const float inv_span = span ? 1.0f / (float)span : 0.0f;
         // Flagging the candidates that surely pass the cone test pays once a voxel's
         // lists serve four passes or more (one pass per list: 7 % slower with it).
-        const bool flag_sure = P.pair == 1 && P.n_sv * P.n_sc >= 128;
+        const bool flag_sure = !FEW && P.n_sv * P.n_sc >= 128;
         for (int vl = 0; vl < tv; vl += VP) {
             // voxel u of the group is brick voxel vl + u; lane u (and every eighth lane after it) holds it
             auto vox_of = [&](int u, int& x, int& y, int& z) {
@@ -1143,7 +1158,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                                     rec = P.rec_out + ((long long)rec_slot * P.n_sv * P.n_sc + (long long)(s0 + j) * P.n_sc + c) *
                                                           kRecWords;
                                 }
-                                const float v = trace_ray<RECORD>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
+                                const float v = trace_ray<RECORD, FEW>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
                                                                   P.status, pc_cry, pc_hole, pc_cone);
                                 if (P.counters) ++cnt_rays;
                                 // Kahan summation of the lane's rays.
@@ -1204,13 +1219,13 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
     }
 }
 
-template <bool RECORD>
+template <bool RECORD, bool FEW>
 __global__ void __launch_bounds__(kPeThreads, 2) pe_trace_kernel(const __grid_constant__ PEParams P,
                                                                 const __grid_constant__ DevGeometry G) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PeSmem& S = *reinterpret_cast<PeSmem*>(smem_raw);
     const long long tile = P.tile_list ? P.tile_list[blockIdx.x] : (long long)blockIdx.x;
-    pe_tile<RECORD>(P, G, S, tile);
+    pe_tile<RECORD, FEW>(P, G, S, tile);
 }
 
 // The batch's geometries, in constant memory: the tile code reads launch
@@ -1245,7 +1260,8 @@ __global__ void __launch_bounds__(kPeThreads, 2) pe_batch_kernel(int n_geoms, lo
         const long long item = s_item;
         const int g = s_geom;
         if (item >= total) break;
-        pe_tile<false>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
+        if (c_batch[g].P.pair > 1) pe_tile<false, true>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
+        else pe_tile<false, false>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
         __syncthreads();
     }
 }
@@ -1257,7 +1273,7 @@ size_t pe_smem_bytes() { return sizeof(PeSmem); }
 // The dynamic shared memory limit is a per-device function attribute: set it
 // once per (device, kernel).
 static cudaError_t allow_smem(const void* fn, int which) {
-    static unsigned long long done[3] = {0, 0, 0};
+    static unsigned long long done[4] = {0, 0, 0, 0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1271,15 +1287,14 @@ cudaError_t pe_launch(const PEParams& p, const DevGeometry& geo, bool record, lo
     const size_t smem = sizeof(PeSmem);
     if (n_tiles <= 0) return cudaSuccess;
     if (n_tiles > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if (record) {
-        cudaError_t e = allow_smem((const void*)pe_trace_kernel<true>, 0);
-        if (e != cudaSuccess) return e;
-        pe_trace_kernel<true><<<(unsigned)n_tiles, kPeThreads, smem, stream>>>(p, geo);
-    } else {
-        cudaError_t e = allow_smem((const void*)pe_trace_kernel<false>, 1);
-        if (e != cudaSuccess) return e;
-        pe_trace_kernel<false><<<(unsigned)n_tiles, kPeThreads, smem, stream>>>(p, geo);
-    }
+    auto launch = [&](auto kernel, int which) -> cudaError_t {
+        const cudaError_t e = allow_smem((const void*)kernel, which);
+        if (e == cudaSuccess) kernel<<<(unsigned)n_tiles, kPeThreads, smem, stream>>>(p, geo);
+        return e;
+    };
+    const cudaError_t e = record ? launch(pe_trace_kernel<true, false>, 0)
+                                 : (p.pair > 1 ? launch(pe_trace_kernel<false, true>, 3) : launch(pe_trace_kernel<false, false>, 1));
+    if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
 

@@ -305,14 +305,31 @@ SM_HD float near_div(float a, float b, float rb) {
     return fmaf(fmaf(-q, b, a), rb, q);
 }
 
-SM_HD float near_sqrt(float x) {
-#ifdef __CUDA_ARCH__
-    const float r = rsqrtf(x);
-#else
-    const float r = 1.0f / std::sqrt(x);
-#endif
+SM_HD float near_root(float x, float r) {   // r ~ 1 / sqrt(x)
     const float s = x * r;
     return fmaf(fmaf(-s, s, x), 0.5f * r, s);
+}
+
+SM_HD float near_sqrt(float x) {
+#ifdef __CUDA_ARCH__
+    return near_root(x, rsqrtf(x));
+#else
+    return near_root(x, 1.0f / std::sqrt(x));
+#endif
+}
+
+// chord_through's own value, operation for operation, for a segment a -> b that a
+// filter called a clear chord of the box of half sizes h about the origin; ix, iy,
+// iz and inv_len: the reciprocals of its extents and length, to a few units of 2^-24.
+SM_HD float chord_value(float xi, float yi, float zi, float xo, float yo, float zo, float hx, float hy, float hz,
+                        float ix, float iy, float iz, float inv_len) {
+    const float dx = xo - xi, dy = yo - yi, dz = zo - zi;
+    const float t = near_root(dx * dx + dy * dy + dz * dz, inv_len);
+    const float qx = near_div(t, dx, ix), qy = near_div(t, dy, iy), qz = near_div(t, dz, iz);
+    const float x1 = (-hx - xi) * qx, x2 = (hx - xi) * qx, y1 = (-hy - yi) * qy, y2 = (hy - yi) * qy;
+    const float z1 = (-hz - zi) * qz, z2 = (hz - zi) * qz;
+    return fminf(fminf(fmaxf(x1, x2), fmaxf(y1, y2)), fmaxf(z1, z2)) -
+           fmaxf(fmaxf(fminf(x1, x2), fminf(y1, y2)), fminf(z1, z2));
 }
 
 // chord_hole of a hole cylinder for a segment that runs towards larger y and

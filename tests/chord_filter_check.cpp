@@ -1,7 +1,8 @@
 // Compares the tracer's chord_quick, chord_filter and hole_filter with the reference-order
 // chord_through and chord_hole on the host: chord_filter_check SEED COUNT RANGE.
 // Prints "<wrong calls> <clear hits> <clear misses> <unclear> <largest value error>
-// <holes called missed> <holes called crossed> <of them with another value>".
+// <holes called missed> <holes called crossed> <of them with another value>
+// <crossed boxes with another chord_value>".
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -19,7 +20,7 @@ int main(int argc, char** argv) {
     auto U = [&](float a, float b) { return std::uniform_real_distribution<float>(a, b)(gen); };
     auto side = [&](float h) { return U(0, 1) < 0.5f ? -h : h; };
     const float lat = 0.35f * range;   // image and detector half width; depth up to half the range
-    long wrong = 0, hits = 0, misses = 0, unclear = 0, hole_misses = 0, hole_hits = 0, hole_other = 0;
+    long wrong = 0, hits = 0, misses = 0, unclear = 0, hole_misses = 0, hole_hits = 0, hole_other = 0, other = 0;
     double worst = 0.0;
     for (long i = 0; i < n; ++i) {
         const float hx = U(0.3f, 2), hy = U(0.3f, 4), hz = U(0.3f, 2), near = 3 * delta;
@@ -50,11 +51,13 @@ int main(int argc, char** argv) {
         const float dx = qx - px, dy = qy - py, dz = qz - pz, len = std::sqrt(dx * dx + dy * dy + dz * dz);
         const ChordRay r = make_chord_ray(px, py, pz, dx, dy, dz, len, delta);
         const Box3 box{-hx, -hy, -hz, hx, hy, hz};
-        float chord = 0, quick = 0, ref;
+        float chord = 0, quick = 0, value = 0, ref;
         int f, fq;
         if (i % 3) {
             f = r.ok ? chord_filter(r, kx, ky, kz, hx, hy, hz, delta, &chord) : -1;
             fq = r.ok ? chord_quick(r, kx, ky, kz, hx, hy, hz, &quick) : -1;
+            value = chord_value(px - kx, py - ky, pz - kz, qx - kx, qy - ky, qz - kz, hx, hy, hz, r.ix, r.iy, r.iz,
+                                1 / len);
             ref = chord_through(px - kx, py - ky, pz - kz, qx - kx, qy - ky, qz - kz, box);
         } else {
             const float a = U(-0.5f, 0.5f), c = std::cos(a), s = std::sin(a), ax = px - kx, az = pz - kz;
@@ -62,6 +65,8 @@ int main(int argc, char** argv) {
                                               fmaf(dx, s, dz * c), len, 2 * delta);
             f = k.ok ? chord_filter(k, 0, 0, 0, hx, hy, hz, 2 * delta, &chord) : -1;
             fq = k.ok ? chord_quick(k, 0, 0, 0, hx, hy, hz, &quick) : -1;
+            value = chord_value(ax * c - az * s, py - ky, ax * s + az * c, (qx - kx) * c - (qz - kz) * s, qy - ky,
+                                (qx - kx) * s + (qz - kz) * c, hx, hy, hz, k.ix, k.iy, k.iz, 1 / len);
             ref = chord_through(ax * c - az * s, py - ky, ax * s + az * c, (qx - kx) * c - (qz - kz) * s, qy - ky,
                                 (qx - kx) * s + (qz - kz) * c, box);
         }
@@ -70,7 +75,8 @@ int main(int argc, char** argv) {
         else if (f == 0) { ++misses; wrong += ref != 0; }
         else {
             ++hits;
-            wrong += ref == 0;
+            wrong += ref == 0 || std::fabs(value - ref) > 1e-6f * len;
+            other += value != ref;
             worst = std::fmax(worst, std::fabs((double)chord - ref) / (delta * len * std::fmax(r.ax, std::fmax(r.ay, r.az))));
         }
         // a hole of radius hx between ky - hy and ky + hy; every other one has its wall near the ray
@@ -91,6 +97,6 @@ int main(int argc, char** argv) {
             wrong += (hf == 0 && hr != 0) || (hf == 1 && (hr == 0 || std::fabs(hc - hr) > 2e-6f * len));
         }
     }
-    std::printf("%ld %ld %ld %ld %.3g %ld %ld %ld\n", wrong, hits, misses, unclear, worst, hole_misses, hole_hits, hole_other);
+    std::printf("%ld %ld %ld %ld %.3g %ld %ld %ld %ld\n", wrong, hits, misses, unclear, worst, hole_misses, hole_hits, hole_other, other);
     return 0;
 }
