@@ -27,7 +27,7 @@ namespace smb {
 
 constexpr int kKnNodes = 512;            // Klein-Nishina table: nodes j * pi / 512, j = 0..512
 constexpr int kScTileD = 32;             // detectors per CTA (one per lane)
-constexpr int kScBrickX = 8;             // voxel brick: 8 (x) x 32 (y) x 1 (z); one x column per warp
+constexpr int kScBrickX = 8;             // voxel brick: 8 (x) x 32 (y) x 1 (z); a CTA takes 8, 4, 2 or 1 of its columns
 constexpr int kScBrickY = 32;
 constexpr int kScWarps = 8;
 constexpr int kScThreads = 32 * kScWarps;
@@ -162,7 +162,4 @@ cudaError_t launch_scatter_transfer(const ScatterParams& P, const DevGeometry& G
                                     long long anchor_stride, cudaStream_t s);
 cudaError_t launch_scatter_main(const ScatterParams& P, const DevGeometry& G, const ScatterTables& T,
                                 cudaStream_t s);
-// Crystal kind only, for row lists of scattered detectors (voxels on the lanes); same results.
-cudaError_t launch_scatter_rows(const ScatterParams& P, const DevGeometry& G, const ScatterTables& T, cudaStream_t s);
-
 }  // namespace smb

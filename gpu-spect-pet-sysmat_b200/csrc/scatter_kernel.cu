@@ -336,7 +336,7 @@ __global__ void scatter_transfer_kernel(ScatterParams P, DevGeometry G, ScatterT
 #pragma unroll
                     for (int j = 0; j < kMaxAnchorsPerPass; ++j)
                         if (use[j])
-                            acc[j] += scatter_term(P, D, C, kn, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
+                            acc[j] += scatter_term<false>(P, D, C, kn, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
                                                    Is[j].z);
                 }
             }
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(kTrRanks * kTrSrcs) scatter_transfer_tiled_ker
 #pragma unroll
                 for (int j = 0; j < kMaxAnchorsPerPass; ++j)
                     if (use[j])
-                        acc[j] += scatter_term(P, D, C, kn, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
+                        acc[j] += scatter_term<false>(P, D, C, kn, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
                                                Is[j].z);
             }
         }
@@ -426,292 +426,333 @@ __global__ void __launch_bounds__(kTrRanks * kTrSrcs) scatter_transfer_tiled_ker
     }
 }
 
+// ---- exact scatter of a detector tile and a voxel brick -----------------------------------
+// CTA = 32 detectors x C columns (C = 8, 4, 2 or 1) of 32 voxels along y, 8 warps; 8 / C
+// warps share a column and take every (8 / C)-th detector.  Only a few per cent of the
+// (detector, voxel, scatter point) terms pass the energy window, scattered over lanes, and
+// a term costs some 500 instructions: each warp lists the pairs that can pass and evaluates
+// full warps of them.  Per batch of NQ scatter points:
+//  1. the CTA stages, per (point, detector), everything the terms need of it (Src: offsets,
+//     corner directions, the pair sums), once for all columns, culls the detectors whose
+//     window no voxel of a column reaches, and stages the points' weights (PE of the
+//     source, or the hole's solid angle) per voxel; the loads of the next batch are issued
+//     before the terms of this one;
+//  2. each warp tests its voxels (lane = voxel) for every remaining detector with the
+//     cosine alone against the detector's threshold (margin 2e-3, far above the test's
+//     rounding) and appends the passing (point, detector, voxel) to its queue;
+//  3. whenever 32 entries wait, one term per lane; the sums are doubles in shared memory,
+//     every cell owned by one warp and added to in (source, point) order, so the split
+//     into columns, rows lists and bricks changes no bit.
+// What bounds it: instruction issue (FP32 and transcendental), 2 CTAs of 8 warps per SM by
+// registers and shared memory alike.
+template <int C>
+struct ScShape {
+    static constexpr int NQ = C == 8 ? 4 : 8;          // points per batch (shared memory: 5 KB each)
+    static constexpr int W = kScWarps / C;             // warps per column
+    static constexpr int PER = NQ * 32 * C / kScThreads;   // staged weights per thread
+};
+
+template <int C>
 struct __align__(16) ScSmem {
     KnNode kn[kKnNodes + 1];
-    double acc[kScBrickX][kScBrickY][kScTileD];
-    float4 vox[kScBrickX][kScBrickY];          // voxel centres (world); w < 0 marks outside the grid
-    float pe[kScBrickY][kScBrickX];
-    float scale[kScTileD];                     // per detector: mu_c / mu_pe / points, or plate mu_c / mu_t
-};
-
-template <int KIND>
-__global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(ScatterParams P, DevGeometry G, ScatterTables T) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ScSmem& S = *reinterpret_cast<ScSmem*>(smem_raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int b = blockIdx.x % P.n_bricks;
-    const int dt = blockIdx.x / P.n_bricks;
-    const BrickCol mycol = brick_column(P, b, warp);        // this warp's voxel column
-    const BrickCol stcol = brick_column(P, b, tid & 7);     // the column this thread stages
-    const int y0 = mycol.y0;
-
-    for (int i = tid; i < kKnNodes + 1; i += kScThreads) S.kn[i] = T.kn[i];
-    for (int i = tid; i < kScBrickX * kScBrickY * kScTileD; i += kScThreads) (&S.acc[0][0][0])[i] = 0.0;
-    {
-        const int xx = tid & 7, yy = tid >> 3;
-        const int x = stcol.x, y = y0 + yy;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-        if (stcol.valid && y < P.ny) {
-            const float3 w = voxel_world(P, (float)x, (float)y, (float)stcol.z);
-            v = make_float4(w.x, w.y, w.z, 1.0f);
-        }
-        S.vox[xx][yy] = v;
-    }
-
-    const int rank = P.rank0 + dt * kScTileD + lane;
-    const int d = rank < P.rank1 ? P.perm[rank] : -1;
-    Det D;
-    D.on = false;
-    float scale = 0.0f;
-    if (rank < P.rank1) scale = setup_det<KIND>(P, G, T, d, D);
-    if (warp == 0) S.scale[lane] = scale;
-    __syncthreads();
-
-    const float inv_norm = T.kn_inv_norm;
-    // this warp's voxel column: I0 + t e, t in [0, col_t] (image y axis, rotated)
-    const float4 col0 = S.vox[warp][0];
-    const float col_ex = -P.sin_a, col_ey = P.cos_a;
-    const float col_t = (float)(min(kScBrickY, P.ny - y0) - 1) * P.vy;
-    if (KIND == kScatterCrystal) {
-        const uint32_t* srcw = P.brick_sources + (long long)b * P.src_words;
-        for (int wd = 0; wd < P.src_words; ++wd) {
-            uint32_t bits = srcw[wd];
-            while (bits) {
-                const int s = (wd << 5) + __ffs(bits) - 1;
-                bits &= bits - 1u;
-                __syncthreads();
-                {
-                    const int xx = tid & 7, yy = tid >> 3;
-                    float v = 0.0f;
-                    if (stcol.valid && y0 + yy < P.ny)
-                        v = __ldg(P.pe + (long long)s * P.ld_pe + stcol.x +
-                                  (long long)P.nx * ((y0 + yy) + (long long)P.ny * stcol.z));
-                    S.pe[yy][xx] = v;
-                }
-                __syncthreads();
-                const float my_pe = S.pe[lane][warp];
-                const unsigned live = __ballot_sync(0xffffffffu, my_pe != 0.0f);
-                if (!live) continue;
-                for (int p = 0; p < T.n_points; ++p) {
-                    const int q = s * T.n_points + p;
-                    const float4 src = T.crystal_src[q];
-                    Src C;
-                    bool on = D.on && s != d;
-                    if (on) {
-                        make_src_basic(D, src, C);
-                        // no voxel of the column passes the window cut: the lane sits out
-                        on = column_max_cos(C, col0.x, col0.y, col0.z, col_ex, col_ey, 0.0f, col_t) > D.c_cut;
-                    }
-                    if (!__any_sync(0xffffffffu, on)) continue;
-                    if (on) {
-                        const long long pc = P.pair_col ? P.pair_col[rank] : rank - P.pair_r0;
-                        make_src_rest(D, P.pair[(long long)q * P.pair_ld + pc], C);
-                    }
-                    unsigned m = live;
-                    while (m) {
-                        const int j = __ffs(m) - 1;
-                        m &= m - 1u;
-                        const float w = __shfl_sync(0xffffffffu, my_pe, j);
-                        if (!on) continue;
-                        const float4 I = S.vox[warp][j];
-                        const float isx = (I.x - D.x) * D.cm - (I.z - D.z) * D.sm;
-                        const float isy = I.y - D.y;
-                        const float isz = (I.x - D.x) * D.sm + (I.z - D.z) * D.cm;
-                        const float t = scatter_term(P, D, C, S.kn, inv_norm, I.x, I.y, I.z, isx, isy, isz);
-                        S.acc[warp][j][lane] += (double)(w * t);
-                    }
-                }
-            }
-        }
-    } else {
-        for (int h = 0; h < T.n_holes0; ++h) {
-            const float4 src = T.hole_src[h];
-            Src C;
-            bool on = D.on && mycol.valid;
-            if (on) {
-                make_src_basic(D, src, C);
-                on = column_max_cos(C, col0.x, col0.y, col0.z, col_ex, col_ey, 0.0f, col_t) > D.c_cut;
-            }
-            if (!on) continue;
-            make_src_rest(D, P.pair[(long long)h * P.pair_ld + (rank - P.pair_r0)], C);
-            for (int j = 0; j < kScBrickY; ++j) {
-                const float4 I = S.vox[warp][j];
-                if (I.w < 0.0f) break;
-                // virtual solid angle of the hole seen from the voxel (scatter.cu:1707-1713)
-                const float vr = 0.1f;
-                const float dx = I.x - src.x, dy = I.y - src.y, dz = I.z - src.z;
-                const float L2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                const float Lih = sqrtf(L2);
-                const float w = (vr * vr * 3.14159265358979323846f + src.w * vr) /
-                                (4.0f * 3.14159265358979323846f * L2) * fabsf(src.y - I.y) / Lih;
-                const float isx = (I.x - D.x) * D.cm - (I.z - D.z) * D.sm;
-                const float isy = I.y - D.y;
-                const float isz = (I.x - D.x) * D.sm + (I.z - D.z) * D.cm;
-                const float t = scatter_term(P, D, C, S.kn, inv_norm, I.x, I.y, I.z, isx, isy, isz);
-                S.acc[warp][j][lane] += (double)(w * t);
-            }
-        }
-    }
-    __syncthreads();
-
-    // write the tile: (detector, y, 8 x) with x fastest
-    const int n_rows = min(kScTileD, P.rank1 - (P.rank0 + dt * kScTileD));
-    for (int i = tid; i < n_rows * kScBrickY * kScBrickX; i += kScThreads) {
-        const int xx = i & 7, yy = (i >> 3) & 31, dl = i >> 8;
-        const BrickCol oc = brick_column(P, b, xx);
-        const int yv = y0 + yy;
-        if (!oc.valid || yv >= P.ny) continue;
-        const int rk = P.rank0 + dt * kScTileD + dl;
-        const int dd = P.perm[rk];
-        const float sc = S.scale[dl];
-        const long long col = P.cols ? (long long)oc.ci * P.ny + yv
-                                     : (long long)oc.x + (long long)P.nx * (yv + (long long)P.ny * oc.z);
-        const long long orow = P.slot ? (long long)P.slot[rk] : (long long)(dd - P.dst_row0);
-        float* out = P.dst + orow * P.ld + col;
-        const float v = (float)S.acc[xx][yy][dl] * sc;
-        *out = P.accumulate ? *out + v : v;
-    }
-}
-
-// ---- crystal scatter for scattered detector rows: voxels on the lanes ----------------------
-// The same entries and the same sums as scatter_main_kernel<crystal> (per
-// entry the terms are added in the same (source, point) order, so results are
-// bit-identical), for row lists whose 32 detectors per tile lie far apart: a
-// warp is one voxel column; per source point one lane per detector runs the
-// column's window cull, then the (passing detector, voxel with PE != 0) pairs
-// are spread over the 32 lanes, so lanes are not left idle by detectors that
-// cull or voxels the source does not see.
-// Position of the n-th (from 0) set bit of m; m must have more than n set bits.
-__device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
-    for (int i = 0; i < n; ++i) m &= m - 1u;
-    return __ffs(m) - 1;
-}
-
-struct __align__(16) ScRowSmem {
-    KnNode kn[kKnNodes + 1];
-    double acc[kScBrickX][kScBrickY][kScTileD];
-    float4 vox[kScBrickX][kScBrickY];
-    float pe[kScBrickY][kScBrickX];
-    float scale[kScTileD];
-    Det det[kScTileD];
+    double acc[C][kScTileD][kScBrickY];                // cell (d, y) at [d][y ^ d]: no bank conflicts either way
+    float4 vox[C][kScBrickY];                          // voxel centres (world); w < 0 marks outside the grid
+    float wgt[ScShape<C>::NQ][C][kScBrickY];           // weight of the point for the voxel
+    float4 src[ScShape<C>::NQ];                        // scatter points
+    float4 b[ScShape<C>::NQ][kScTileD];                // D - S, and c_cut |D - S| (1e30: detector off)
+    float4 pr[ScShape<C>::NQ][kScTileD];               // pair sums
+    float4 e[ScShape<C>::NQ][8][kScTileD];             // corner directions; w: |D-S|^2, |D-S|, phi_k, c_len, S in D's frame
+    float4 det[4][kScTileD];                           // Det's fields
+    float scale[kScTileD];                             // per detector: mu_c / mu_pe / points, or plate mu_c / mu_t
     int d[kScTileD];
-    long long pc[kScTileD];                    // pair column of each detector
+    unsigned todo[ScShape<C>::NQ][C];                  // per (point, column): detectors that pass the column's cull
+    unsigned short queue[kScWarps][64];                // point << 10 | detector << 5 | voxel
 };
 
-__global__ void __launch_bounds__(kScThreads, 2) scatter_rows_kernel(ScatterParams P, DevGeometry G, ScatterTables T) {
+template <int C>
+constexpr bool two_ctas() { return 2 * (sizeof(ScSmem<C>) + 1024) <= 228 * 1024; }
+static_assert(two_ctas<8>() && two_ctas<4>() && two_ctas<2>() && two_ctas<1>(), "two CTAs per SM");
+
+// scatter_term's view of a staged (point, detector).
+struct SrcView {
+    const float4* e;             // [8] corner directions, stride kScTileD
+    float sx, sy, sz, ssx, ssy, ssz, bx, by, bz, bb, L, phi_k, c_len;
+    float4 pr;
+    __device__ __forceinline__ float3 corner(int i) const {
+        const float4 v = e[i * kScTileD];
+        return make_float3(v.x, v.y, v.z);
+    }
+    __device__ __forceinline__ float3 pick(int i) const { return corner(i); }
+};
+
+template <int KIND, int C>
+__global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __grid_constant__ ScatterParams P,
+                                                                    const __grid_constant__ DevGeometry G,
+                                                                    const __grid_constant__ ScatterTables T) {
+    using Shape = ScShape<C>;
+    constexpr int NQ = Shape::NQ, W = Shape::W, PER = Shape::PER, PARTS = kScBrickX / C;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    ScRowSmem& S = *reinterpret_cast<ScRowSmem*>(smem_raw);
+    ScSmem<C>& S = *reinterpret_cast<ScSmem<C>*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int b = blockIdx.x % P.n_bricks;
-    const int dt = blockIdx.x / P.n_bricks;
-    const BrickCol mycol = brick_column(P, b, warp);
-    const BrickCol stcol = brick_column(P, b, tid & 7);
-    const int y0 = mycol.y0;
+    const int part = blockIdx.x % PARTS, b = (blockIdx.x / PARTS) % P.n_bricks, dt = blockIdx.x / (PARTS * P.n_bricks);
+    const int c0 = part * C;                                 // first column of the brick
+    const int y0 = brick_column(P, b, 0).y0;
 
     for (int i = tid; i < kKnNodes + 1; i += kScThreads) S.kn[i] = T.kn[i];
-    for (int i = tid; i < kScBrickX * kScBrickY * kScTileD; i += kScThreads) (&S.acc[0][0][0])[i] = 0.0;
-    {
-        const int xx = tid & 7, yy = tid >> 3;
-        const int x = stcol.x, y = y0 + yy;
+    for (int i = tid; i < C * kScBrickY * kScTileD; i += kScThreads) (&S.acc[0][0][0])[i] = 0.0;
+    for (int i = tid; i < C * kScBrickY; i += kScThreads) {
+        const BrickCol bc = brick_column(P, b, c0 + i % C);
+        const int y = y0 + i / C;
         float4 v = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-        if (stcol.valid && y < P.ny) {
-            const float3 w = voxel_world(P, (float)x, (float)y, (float)stcol.z);
+        if (bc.valid && y < P.ny) {
+            const float3 w = voxel_world(P, (float)bc.x, (float)y, (float)bc.z);
             v = make_float4(w.x, w.y, w.z, 1.0f);
         }
-        S.vox[xx][yy] = v;
+        S.vox[i % C][i / C] = v;
     }
+    const int n_det = min(kScTileD, P.rank1 - (P.rank0 + dt * kScTileD));
     if (warp == 0) {
         const int rank = P.rank0 + dt * kScTileD + lane;
-        Det D;
+        Det D{};
         D.on = false;
         float scale = 0.0f;
         int d = -1;
-        if (rank < P.rank1) {
+        if (lane < n_det) {
             d = P.perm[rank];
-            scale = setup_det<kScatterCrystal>(P, G, T, d, D);
+            scale = setup_det<KIND>(P, G, T, d, D);
         }
-        S.det[lane] = D;
-        S.d[lane] = d;
+        S.det[0][lane] = make_float4(D.x, D.y, D.z, D.cm);
+        S.det[1][lane] = make_float4(D.sm, D.hw, D.ht, D.hh);
+        S.det[2][lane] = make_float4(D.r_unit, D.mu_pe, D.mu_c, D.res);
+        S.det[3][lane] = make_float4(D.lo, D.hi, D.on ? D.c_cut : 2.0f, 0.0f);
         S.scale[lane] = scale;
-        S.pc[lane] = rank < P.rank1 ? (P.pair_col ? (long long)P.pair_col[rank] : (long long)(rank - P.pair_r0)) : 0;
+        S.d[lane] = d;
     }
     __syncthreads();
-    const int n_det = min(kScTileD, P.rank1 - (P.rank0 + dt * kScTileD));
 
-    const float inv_norm = T.kn_inv_norm;
-    const float4 col0 = S.vox[warp][0];
+    // this warp's column: I0 + t e, t in [0, col_t] (image y axis, rotated); lane = voxel
+    const int col = warp / W, sub = warp % W;
+    const float4 I = S.vox[col][lane];
     const float col_ex = -P.sin_a, col_ey = P.cos_a;
     const float col_t = (float)(min(kScBrickY, P.ny - y0) - 1) * P.vy;
-    const uint32_t* srcw = P.brick_sources + (long long)b * P.src_words;
-    for (int wd = 0; wd < P.src_words; ++wd) {
-        uint32_t bits = srcw[wd];
-        while (bits) {
-            const int s = (wd << 5) + __ffs(bits) - 1;
-            bits &= bits - 1u;
-            __syncthreads();
-            {
-                const int xx = tid & 7, yy = tid >> 3;
-                float v = 0.0f;
-                if (stcol.valid && y0 + yy < P.ny)
-                    v = __ldg(P.pe + (long long)s * P.ld_pe + stcol.x +
-                              (long long)P.nx * ((y0 + yy) + (long long)P.ny * stcol.z));
-                S.pe[yy][xx] = v;
+    const float c_cut = S.det[3][lane].z;                    // lane = detector
+    const unsigned mine = W == 1 ? 0xffffffffu : (W == 2 ? 0x55555555u : (W == 4 ? 0x11111111u : 0x01010101u)) << sub;
+
+    // This thread's place in the staged weights: one voxel of the tile, points first, first + step, ...
+    constexpr int kPlaces = 32 * C, kStep = kScThreads / kPlaces;
+    const int w_first = tid / kPlaces, w_col = tid % C, w_y = tid % kPlaces / C;
+    long long w_at = -1;
+    if (KIND == kScatterCrystal) {
+        const BrickCol bc = brick_column(P, b, c0 + w_col);
+        if (bc.valid && y0 + w_y < P.ny) w_at = bc.x + (long long)P.nx * (y0 + w_y + (long long)P.ny * bc.z);
+    }
+    long long pair_at = 0;                                   // this lane's pair column
+    if (lane < n_det) {
+        const int rank = P.rank0 + dt * kScTileD + lane;
+        pair_at = P.pair_col ? P.pair_col[rank] : rank - P.pair_r0;
+    }
+
+    // The scatter points in order: sources with PE != 0 in the brick and their points, or the holes.
+    const uint32_t* srcw = KIND == kScatterCrystal ? P.brick_sources + (long long)b * P.src_words : nullptr;
+    int wd = -1, next_p = T.n_points, next_s = -1;
+    uint32_t bits = 0u;
+    // Loads of a batch: weights (crystal kind) and this thread's pair sums.  q: points, -1 past
+    // the last; s: their sources.
+    int q[NQ], s[NQ];
+    float pe[PER];
+    float4 pr;
+    auto fetch = [&] {
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            q[k] = s[k] = -1;
+            if (KIND != kScatterCrystal) {
+                if (next_s + 1 < T.n_holes0) q[k] = ++next_s;
+                continue;
             }
-            __syncthreads();
-            const unsigned live = __ballot_sync(0xffffffffu, S.pe[lane][warp] != 0.0f);
-            if (!live) continue;
-            const int n_live = __popc(live);
-            for (int p = 0; p < T.n_points; ++p) {
-                const int q = s * T.n_points + p;
-                const float4 src = T.crystal_src[q];
-                // window cull of the column, one detector per lane
-                bool pass = false;
-                if (lane < n_det) {
-                    const Det& D = S.det[lane];
-                    if (D.on && s != S.d[lane]) {
-                        Src C;
-                        make_src_basic(D, src, C);
-                        pass = column_max_cos(C, col0.x, col0.y, col0.z, col_ex, col_ey, 0.0f, col_t) > D.c_cut;
-                    }
-                }
-                const unsigned pmask = __ballot_sync(0xffffffffu, pass);
-                if (!pmask) continue;
-                // (passing detector, live voxel) pairs spread over the lanes; each pair once per point
-                const int n_items = __popc(pmask) * n_live;
-                for (int base = 0; base < n_items; base += 32) {
-                    const int item = base + lane;
-                    if (item >= n_items) continue;
-                    const int k = item / n_live, jj = item - k * n_live;
-                    const int dl = nth_set_bit(pmask, k), j = nth_set_bit(live, jj);
-                    const Det& D = S.det[dl];
-                    Src C;
-                    make_src_basic(D, src, C);
-                    make_src_rest(D, P.pair[(long long)q * P.pair_ld + S.pc[dl]], C);
-                    const float4 Iv = S.vox[warp][j];
-                    const float isx = (Iv.x - D.x) * D.cm - (Iv.z - D.z) * D.sm;
-                    const float isy = Iv.y - D.y;
-                    const float isz = (Iv.x - D.x) * D.sm + (Iv.z - D.z) * D.cm;
-                    const float t = scatter_term(P, D, C, S.kn, inv_norm, Iv.x, Iv.y, Iv.z, isx, isy, isz);
-                    S.acc[warp][j][dl] += (double)(S.pe[j][warp] * t);
-                }
+            if (next_p >= T.n_points) {
+                while (!bits && wd + 1 < P.src_words) bits = srcw[++wd];
+                if (!bits) continue;
+                next_s = (wd << 5) + __ffs(bits) - 1;
+                bits &= bits - 1u;
+                next_p = 0;
             }
+            q[k] = next_s * T.n_points + next_p++;
+            s[k] = next_s;
+        }
+        if (KIND == kScatterCrystal) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                int sk = -1;
+#pragma unroll
+                for (int j = 0; j < NQ; ++j) sk = w_first + i * kStep == j ? s[j] : sk;
+                pe[i] = sk >= 0 && w_at >= 0 ? __ldg(P.pe + (long long)sk * P.ld_pe + w_at) : 0.0f;
+            }
+        }
+        pr = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (warp < NQ && lane < n_det) {
+            int qk = -1;
+#pragma unroll
+            for (int j = 0; j < NQ; ++j) qk = warp == j ? q[j] : qk;
+            if (qk >= 0) pr = __ldg(P.pair + (long long)qk * P.pair_ld + pair_at);
+        }
+    };
+    fetch();
+    while (q[0] >= 0) {
+        __syncthreads();                                     // the previous batch's terms are done
+        int n_q = 0;
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) n_q += q[k] >= 0;
+        if (KIND == kScatterCrystal) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) S.wgt[w_first + i * kStep][w_col][w_y] = pe[i];
+        }
+        if (warp < n_q) {
+            int qk = q[0], sk = s[0];
+#pragma unroll
+            for (int j = 1; j < NQ; ++j) {
+                qk = warp == j ? q[j] : qk;
+                sk = warp == j ? s[j] : sk;
+            }
+            const float4 pt = KIND == kScatterCrystal ? T.crystal_src[qk] : T.hole_src[qk];
+            if (lane == 0) S.src[warp] = pt;
+            Det D;
+            const float4 d0 = S.det[0][lane], d1 = S.det[1][lane];
+            D.x = d0.x; D.y = d0.y; D.z = d0.z; D.cm = d0.w; D.sm = d1.x; D.hw = d1.y; D.ht = d1.z; D.hh = d1.w;
+            D.r_unit = S.det[2][lane].x;
+            const bool on = c_cut < 2.0f && !(KIND == kScatterCrystal && sk == S.d[lane]);
+            Src c;
+            make_src_basic(D, pt, c);
+            S.b[warp][lane] = make_float4(c.bx, c.by, c.bz, on ? c_cut * c.L : 1e30f);
+            // detectors whose window no voxel of a column passes sit that column out
+            for (int xx = 0; xx < C; ++xx) {
+                const float4 v0 = S.vox[xx][0];
+                const unsigned m = __ballot_sync(0xffffffffu, on && column_max_cos(c, v0.x, v0.y, v0.z, col_ex, col_ey, 0.0f, col_t) > c_cut);
+                if (lane == 0) S.todo[warp][xx] = m;
+            }
+            if (on) {
+                make_src_rest(D, pr, c);
+                const float more[8] = {c.bb, c.L, c.phi_k, c.c_len, c.ssx, c.ssy, c.ssz, 0.0f};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) S.e[warp][i][lane] = make_float4(c.e[i][0], c.e[i][1], c.e[i][2], more[i]);
+                S.pr[warp][lane] = pr;
+            }
+        }
+        __syncthreads();
+        fetch();                                             // next batch, in flight during the terms
+
+        int count = 0;                                       // queue length
+        int k = 0;                                           // point of the batch
+        unsigned todo = 0u;                                  // its detectors still to test
+        float ax = 0.0f, ay = 0.0f, az = 0.0f, inv_a = 0.0f;
+        bool live = false;
+        auto open_point = [&] {
+            // weights and directions of the voxels (lane)
+            const float4 pt = S.src[k];
+            float w;
+            if (KIND == kScatterCrystal) {
+                w = S.wgt[k][col][lane];
+                live = w != 0.0f;
+            } else {
+                // virtual solid angle of the hole seen from the voxel (scatter.cu:1707-1713)
+                const float vr = 0.1f;
+                const float dx = I.x - pt.x, dy = I.y - pt.y, dz = I.z - pt.z;
+                const float L2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                const float Lih = sqrtf(L2);
+                w = (vr * vr * 3.14159265358979323846f + pt.w * vr) / (4.0f * 3.14159265358979323846f * L2) *
+                    fabsf(pt.y - I.y) / Lih;
+                S.wgt[k][col][lane] = w;                     // (the column's warps write the same values)
+                live = I.w >= 0.0f;
+            }
+            todo = __any_sync(0xffffffffu, live) ? S.todo[k][col] & mine : 0u;
+            ax = pt.x - I.x; ay = pt.y - I.y; az = pt.z - I.z;
+            inv_a = rsqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+        };
+        open_point();
+        for (;;) {
+            // fill the queue to a full warp of terms
+            while (count < 32) {
+                if (!todo) {
+                    if (++k >= n_q) break;
+                    open_point();
+                    continue;
+                }
+                const int dl = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const float4 bd = S.b[k][dl];
+                const bool pass = live && fmaf(ax, bd.x, fmaf(ay, bd.y, az * bd.z)) * inv_a > bd.w;
+                const unsigned m = __ballot_sync(0xffffffffu, pass);
+                if (pass) S.queue[warp][count + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(k << 10 | dl << 5 | lane);
+                count += __popc(m);
+            }
+            if (count == 0) break;
+            __syncwarp();
+            const int n = min(count, 32);
+            const unsigned item = S.queue[warp][lane < n ? lane : 0];
+            const int slot = item >> 10, dl = item >> 5 & 31, j = item & 31;
+            double add = 0.0;
+            if (lane < n) {
+                Det D;
+                const float4 d0 = S.det[0][dl], d1 = S.det[1][dl], d2 = S.det[2][dl], d3 = S.det[3][dl];
+                D.x = d0.x; D.y = d0.y; D.z = d0.z; D.cm = d0.w;
+                D.sm = d1.x; D.hw = d1.y; D.ht = d1.z; D.hh = d1.w;
+                D.r_unit = d2.x; D.mu_pe = d2.y; D.mu_c = d2.z; D.res = d2.w;
+                D.lo = d3.x; D.hi = d3.y;
+                SrcView c;
+                c.e = &S.e[slot][0][dl];
+                const float4 pt = S.src[slot], bd = S.b[slot][dl];
+                c.sx = pt.x; c.sy = pt.y; c.sz = pt.z;
+                c.bx = bd.x; c.by = bd.y; c.bz = bd.z;
+                c.bb = c.e[0].w; c.L = c.e[kScTileD].w; c.phi_k = c.e[2 * kScTileD].w; c.c_len = c.e[3 * kScTileD].w;
+                c.ssx = c.e[4 * kScTileD].w; c.ssy = c.e[5 * kScTileD].w; c.ssz = c.e[6 * kScTileD].w;
+                c.pr = S.pr[slot][dl];
+                const float4 V = S.vox[col][j];
+                const float isx = (V.x - D.x) * D.cm - (V.z - D.z) * D.sm;
+                const float isy = V.y - D.y;
+                const float isz = (V.x - D.x) * D.sm + (V.z - D.z) * D.cm;
+                const float t = scatter_term<true>(P, D, c, S.kn, T.kn_inv_norm, V.x, V.y, V.z, isx, isy, isz);
+                add = (double)(S.wgt[slot][col][j] * t);
+            }
+            // a cell may wait for several points: one point at a time
+            const int last = __shfl_sync(0xffffffffu, slot, n - 1);
+            for (int p = __shfl_sync(0xffffffffu, slot, 0); p <= last; ++p) {
+                if (lane < n && slot == p) S.acc[col][dl][j ^ dl] += add;
+                __syncwarp();
+            }
+            // the rest of the queue moves up
+            const unsigned short rest = S.queue[warp][32 + lane];
+            __syncwarp();
+            if (lane < count - n) S.queue[warp][lane] = rest;
+            count -= n;
         }
     }
     __syncthreads();
-    for (int i = tid; i < n_det * kScBrickY * kScBrickX; i += kScThreads) {
-        const int xx = i & 7, yy = (i >> 3) & 31, dl = i >> 8;
-        const BrickCol oc = brick_column(P, b, xx);
+
+    // write the tile: (detector, y, C columns) with the column fastest
+    for (int i = tid; i < n_det * kScBrickY * C; i += kScThreads) {
+        const int xx = i % C, yy = i / C % kScBrickY, dl = i / (C * kScBrickY);
+        const BrickCol oc = brick_column(P, b, c0 + xx);
         const int yv = y0 + yy;
         if (!oc.valid || yv >= P.ny) continue;
         const int rk = P.rank0 + dt * kScTileD + dl;
-        const int dd = S.d[dl];
-        const long long col = P.cols ? (long long)oc.ci * P.ny + yv
-                                     : (long long)oc.x + (long long)P.nx * (yv + (long long)P.ny * oc.z);
-        const long long orow = P.slot ? (long long)P.slot[rk] : (long long)(dd - P.dst_row0);
-        float* out = P.dst + orow * P.ld + col;
-        const float v = (float)S.acc[xx][yy][dl] * S.scale[dl];
+        const long long ocol = P.cols ? (long long)oc.ci * P.ny + yv
+                                      : (long long)oc.x + (long long)P.nx * (yv + (long long)P.ny * oc.z);
+        const long long orow = P.slot ? (long long)P.slot[rk] : (long long)(S.d[dl] - P.dst_row0);
+        float* out = P.dst + orow * P.ld + ocol;
+        const float v = (float)S.acc[xx][dl][yy ^ dl] * S.scale[dl];
         *out = P.accumulate ? *out + v : v;
     }
+}
+
+template <int KIND, int C>
+cudaError_t launch_main(const ScatterParams& P, const DevGeometry& G, const ScatterTables& T, long long tiles,
+                        cudaStream_t s) {
+    const long long blocks = tiles * (kScBrickX / C);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    const cudaError_t e = cudaFuncSetAttribute(scatter_main_kernel<KIND, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(ScSmem<C>));
+    if (e != cudaSuccess) return e;
+    scatter_main_kernel<KIND, C><<<(unsigned)blocks, kScThreads, sizeof(ScSmem<C>), s>>>(P, G, T);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -792,36 +833,28 @@ cudaError_t launch_scatter_transfer(const ScatterParams& P, const DevGeometry& G
     return cudaGetLastError();
 }
 
-cudaError_t launch_scatter_rows(const ScatterParams& P, const DevGeometry& G, const ScatterTables& T, cudaStream_t s) {
-    const size_t smem = sizeof(ScRowSmem);
-    const long long d_tiles = (P.rank1 - P.rank0 + kScTileD - 1) / kScTileD;
-    const long long blocks = d_tiles * P.n_bricks;
-    if (blocks <= 0) return cudaSuccess;
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(scatter_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    scatter_rows_kernel<<<(unsigned)blocks, kScThreads, smem, s>>>(P, G, T);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_scatter_main(const ScatterParams& P, const DevGeometry& G, const ScatterTables& T,
                                 cudaStream_t s) {
-    const size_t smem = sizeof(ScSmem);
-    const long long d_tiles = (P.rank1 - P.rank0 + kScTileD - 1) / kScTileD;
-    const long long blocks = d_tiles * P.n_bricks;
-    if (blocks <= 0) return cudaSuccess;
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cudaError_t e;
+    const long long tiles = (long long)((P.rank1 - P.rank0 + kScTileD - 1) / kScTileD) * P.n_bricks;
+    if (tiles <= 0) return cudaSuccess;
+    int dev = 0, sms = 148;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    // Fewer columns per CTA repeat the staging and the culls; they pay while the CTAs
+    // would fill less than four waves of the device (2 per SM).
+    const long long want = 8LL * sms;
+    const int c = tiles >= want ? 8 : (2 * tiles >= want ? 4 : (4 * tiles >= want ? 2 : 1));
     if (P.kind == kScatterCrystal) {
-        e = cudaFuncSetAttribute(scatter_main_kernel<kScatterCrystal>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        scatter_main_kernel<kScatterCrystal><<<(unsigned)blocks, kScThreads, smem, s>>>(P, G, T);
-    } else {
-        e = cudaFuncSetAttribute(scatter_main_kernel<kScatterCollimator>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        scatter_main_kernel<kScatterCollimator><<<(unsigned)blocks, kScThreads, smem, s>>>(P, G, T);
+        if (c == 8) return launch_main<kScatterCrystal, 8>(P, G, T, tiles, s);
+        if (c == 4) return launch_main<kScatterCrystal, 4>(P, G, T, tiles, s);
+        if (c == 2) return launch_main<kScatterCrystal, 2>(P, G, T, tiles, s);
+        return launch_main<kScatterCrystal, 1>(P, G, T, tiles, s);
     }
-    return cudaGetLastError();
+    if (c == 8) return launch_main<kScatterCollimator, 8>(P, G, T, tiles, s);
+    if (c == 4) return launch_main<kScatterCollimator, 4>(P, G, T, tiles, s);
+    if (c == 2) return launch_main<kScatterCollimator, 2>(P, G, T, tiles, s);
+    return launch_main<kScatterCollimator, 1>(P, G, T, tiles, s);
 }
 
 }  // namespace smb
