@@ -50,6 +50,7 @@ struct ScatterTables {
     int n_crystals;
     int n_holes0;                // holes of plate 0 (Collimator[10])
     int n_points;                // scatter points per crystal
+    float chord_delta;           // chord_filter's margin for rays from scatter points to crystals
     float kn_inv_norm;           // 1 / (rectangle sum of g over [0, pi], as the reference normalises)
 };
 
@@ -100,6 +101,7 @@ struct HostScatterTables {
     std::vector<KnNode> kn;
     int n_points = 1;
     int sp[3] = {1, 1, 1};
+    float chord_delta = 0.0f;
     float kn_inv_norm = 0.0f;
 };
 
@@ -112,6 +114,7 @@ int64_t collimator_bitmap_words(int n_crystals, int n_holes0);
 cudaError_t launch_bitmap_crystal(uint32_t* words, int64_t n_words, const ScatterTables& T, cudaStream_t s);
 cudaError_t launch_bitmap_collimator(uint32_t* words, int64_t n_words, const ScatterTables& T, cudaStream_t s);
 // pair[q][r - r0] for every source point q of `kind` and detectors perm[r], r in [r0, r1).
+// bitmap: the kind's bitmap, or null: its bits are decided where a crystal is crossed.
 cudaError_t launch_scatter_pairs(int kind, const DevGeometry& G, const ScatterTables& T, const uint32_t* bitmap,
                                  const int* perm, int r0, int r1, float4* pair, cudaStream_t s);
 

@@ -46,6 +46,7 @@ int upload_tables(const HostScatterTables& H, int n_crystals, int n_holes0, cuda
     T->n_crystals = n_crystals;
     T->n_holes0 = n_holes0;
     T->n_points = H.n_points;
+    T->chord_delta = H.chord_delta;
     T->kn_inv_norm = H.kn_inv_norm;
     return SM_OK;
 }
@@ -136,22 +137,8 @@ int exact_scatter(const sm_geometry* geo, const int sp[3], int parts, float angl
         P.n_bricks = P.bricks_x * P.bricks_y;
     }
 
-    DevBuf bm_c, bm_h, bricks, pairs;
-    const uint32_t* bmc = d_bm_crystal;
-    const uint32_t* bmh = d_bm_collimator;
+    DevBuf bricks;
     const bool do_crystal = (parts & 1) != 0, do_collimator = (parts & 2) != 0 && h0 > 0;
-    if (do_crystal && !bmc && !spec.pairs) {
-        const int64_t w = crystal_bitmap_words(N);
-        SM_TRY(bm_c.alloc(sizeof(uint32_t) * (size_t)w, s, "crystal bitmap"));
-        SM_CUDA(launch_bitmap_crystal(static_cast<uint32_t*>(bm_c.p), w, T, s));
-        bmc = static_cast<const uint32_t*>(bm_c.p);
-    }
-    if (do_collimator && !bmh) {
-        const int64_t w = collimator_bitmap_words(N, h0);
-        SM_TRY(bm_h.alloc(sizeof(uint32_t) * (size_t)w, s, "collimator bitmap"));
-        SM_CUDA(launch_bitmap_collimator(static_cast<uint32_t*>(bm_h.p), w, T, s));
-        bmh = static_cast<const uint32_t*>(bm_h.p);
-    }
     bool written = false;
     if (do_crystal) {
         P.src_words = (N + 31) / 32;
@@ -204,7 +191,8 @@ int exact_scatter(const sm_geometry* geo, const int sp[3], int parts, float angl
         SM_TRY(pair.alloc(pb, s, "scatter pairs"));
         for (int c0 = 0; c0 < n_rank; c0 += chunk) {
             const int c1 = std::min(n_rank, c0 + chunk);
-            SM_CUDA(launch_scatter_pairs(kind, geo->dev.view, T, kind == kScatterCrystal ? bmc : bmh, P.perm, c0, c1,
+            SM_CUDA(launch_scatter_pairs(kind, geo->dev.view, T,
+                                         kind == kScatterCrystal ? d_bm_crystal : d_bm_collimator, P.perm, c0, c1,
                                          static_cast<float4*>(pair.p), s));
             ScatterParams Q = P;
             Q.kind = kind;
@@ -242,14 +230,9 @@ int crystal_pair_table(const sm_geometry* geo, const int sp[3], DevBuf* table, s
     *order = spatial_order(g, 0, N);
     SM_TRY(d_order->alloc(sizeof(int) * (size_t)N, s, "detector order"));
     SM_CUDA(cudaMemcpyAsync(d_order->p, order->data(), sizeof(int) * (size_t)N, cudaMemcpyHostToDevice, s));
-    DevBuf bm;
-    const int64_t w = crystal_bitmap_words(N);
-    SM_TRY(bm.alloc(sizeof(uint32_t) * (size_t)w, s, "crystal bitmap"));
-    SM_CUDA(launch_bitmap_crystal(static_cast<uint32_t*>(bm.p), w, T, s));
     const size_t n_src = (size_t)N * T.n_points;
     SM_TRY(table->alloc(sizeof(float4) * n_src * (size_t)N, s, "crystal pair table"));
-    SM_CUDA(launch_scatter_pairs(kScatterCrystal, geo->dev.view, T, static_cast<const uint32_t*>(bm.p),
-                                 static_cast<const int*>(d_order->p), 0, N, static_cast<float4*>(table->p), s));
+    SM_CUDA(launch_scatter_pairs(kScatterCrystal, geo->dev.view, T, nullptr, static_cast<const int*>(d_order->p), 0, N, static_cast<float4*>(table->p), s));
     SM_CUDA(cudaStreamSynchronize(s));   // the host tables are released on return
     return SM_OK;
 }
@@ -279,14 +262,11 @@ int scatter_transfer(const sm_geometry* geo, const int sp[3], float angle, const
     }
     std::vector<int> ident(N);
     for (int i = 0; i < N; ++i) ident[i] = i;
-    DevBuf perm, bm;
+    DevBuf perm;
     SM_TRY(perm.alloc(sizeof(int) * (size_t)N, s, "detector order"));
     SM_CUDA(cudaMemcpyAsync(perm.p, ident.data(), sizeof(int) * (size_t)N, cudaMemcpyHostToDevice, s));
     SM_CUDA(cudaStreamSynchronize(s));
     P.perm = static_cast<const int*>(perm.p);
-    const int64_t w = crystal_bitmap_words(N);
-    SM_TRY(bm.alloc(sizeof(uint32_t) * (size_t)w, s, "crystal bitmap"));
-    SM_CUDA(launch_bitmap_crystal(static_cast<uint32_t*>(bm.p), w, T, s));
     const int n_src = N * T.n_points;
     int chunk = (int)std::max<size_t>(128, kPairBudget / (sizeof(float4) * (size_t)std::max(1, n_src)));
     chunk = std::max(128, chunk / 128 * 128);
@@ -294,7 +274,7 @@ int scatter_transfer(const sm_geometry* geo, const int sp[3], float angle, const
     SM_TRY(pair.alloc(sizeof(float4) * (size_t)n_src * (size_t)std::min(chunk, N), s, "scatter pairs"));
     for (int c0 = 0; c0 < N; c0 += chunk) {
         const int c1 = std::min(N, c0 + chunk);
-        SM_CUDA(launch_scatter_pairs(kScatterCrystal, geo->dev.view, T, static_cast<const uint32_t*>(bm.p), P.perm, c0, c1,
+        SM_CUDA(launch_scatter_pairs(kScatterCrystal, geo->dev.view, T, nullptr, P.perm, c0, c1,
                                      static_cast<float4*>(pair.p), s));
         ScatterParams Q = P;
         Q.rank0 = c0;

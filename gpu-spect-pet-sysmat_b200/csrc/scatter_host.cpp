@@ -184,6 +184,16 @@ int build_scatter_tables(const HostGeometry& g, const int sp[3], HostScatterTabl
         s[2] = H[3];
         s[3] = H[2] - H[1];
     }
+    // coordinate range of the rays: the crystals and the holes
+    float lo[3], hi[3], s2 = 0.0f;
+    for (int a = 0; a < 3; ++a) lo[a] = g.lo[a], hi[a] = g.hi[a];
+    for (int i = 0; i < h0; ++i)
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = std::min(lo[a], T.hole_src[4 * (size_t)i + a]);
+            hi[a] = std::max(hi[a], T.hole_src[4 * (size_t)i + a]);
+        }
+    for (int a = 0; a < 3; ++a) s2 += (hi[a] - lo[a]) * (hi[a] - lo[a]);
+    T.chord_delta = 1.5e-6f * std::sqrt(s2);
     build_kn_table(g.physics[7], &T.kn, &T.kn_inv_norm);
     return SM_OK;
 }

@@ -38,7 +38,7 @@ __device__ __forceinline__ float dist3(float x1, float y1, float z1, float x2, f
     return sqrtf((x1 - x2) * (x1 - x2) + (y1 - y2) * (y1 - y2) + (z1 - z2) * (z1 - z2));
 }
 
-__device__ bool crystal_bit(const float4* cr, int i, int j, int k) {
+__device__ __noinline__ bool crystal_bit(const float4* cr, int i, int j, int k) {
     const float4 a = cr[i], b = cr[j], c = cr[k];
     const float Lij = dist3(a.x, a.y, a.z, b.x, b.y, b.z);
     const float crit_ij = a.w / Lij, crit_ji = b.w / Lij;
@@ -54,7 +54,7 @@ __device__ bool crystal_bit(const float4* cr, int i, int j, int k) {
     return dist3(ex_kj, ey_kj, ez_kj, ex_ij, ey_ij, ez_ij) <= crit_kj + crit_ij;
 }
 
-__device__ bool collimator_bit(const float4* cr, const float4* hr, int i, int j, int k) {
+__device__ __noinline__ bool collimator_bit(const float4* cr, const float4* hr, int i, int j, int k) {
     const float4 h = hr[i], b = cr[j], c = cr[k];
     const float Lij = dist3(h.x, h.y, h.z, b.x, b.y, b.z);
     const float crit_ji = b.w / Lij;
@@ -76,56 +76,102 @@ __device__ __forceinline__ int pair_row(long long pair, int N) {
     return i;
 }
 
-// One thread per 32-bit word: bits bit0 .. bit0 + 31 of the pair-major bitmap
-// bit = (i N - i (i + 1) / 2 + j) N + k, i <= j; set for i < j, k != i, j.
-__global__ void bitmap_crystal_kernel(uint32_t* words, long long n_words, ScatterTables T) {
-    const int N = T.n_crystals;
-    const long long total = ((long long)N * (N + 1) / 2) * N;
-    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < n_words;
-         w += (long long)gridDim.x * blockDim.x) {
-        const long long bit0 = w * 32;
-        long long pair = bit0 / N;
-        int k = (int)(bit0 - pair * N);
-        int i = pair_row(pair, N);
-        int j = (int)(pair - ((long long)i * N - (long long)i * (i - 1) / 2)) + i;
-        uint32_t word = 0u;
-        for (int b = 0; b < 32 && bit0 + b < total; ++b) {
-            if (i < j && k != i && k != j && crystal_bit(T.crystal_raw, i, j, k)) word |= 1u << b;
-            if (++k == N) {
-                k = 0;
-                if (++j == N) {
-                    ++i;
-                    j = i;
-                }
-            }
-        }
-        words[w] = word;
-    }
+// The cone test |u_k - u_axis| <= R_k / |k - a| + c (u_k, u_axis unit vectors from a) by
+// squares with one reciprocal square root: 1 yes, 0 no, -1 too close to call.  The
+// squared distance 2 - 2 cos is good to 2e-6 and the right side to 1e-6 of itself, the
+// band is five times that and more.
+__device__ __forceinline__ int cone_quick(const float4& k, float ax, float ay, float az, float ux, float uy, float uz,
+                                          float c) {
+    const float dx = k.x - ax, dy = k.y - ay, dz = k.z - az;
+    const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+    const float cosine = fmaf(dx, ux, fmaf(dy, uy, dz * uz)) * inv;
+    const float rhs = fmaf(k.w, inv, c), r2 = rhs * rhs;
+    const float diff = fmaf(-2.0f, cosine, 2.0f) - r2, band = fmaf(1e-4f, r2, 1e-5f);
+    return diff < -band ? 1 : (diff > band ? 0 : -1);
 }
 
-// bit = i N^2 + j N + k for layer-0 hole i, crystals j, k.
-__global__ void bitmap_collimator_kernel(uint32_t* words, long long n_words, ScatterTables T) {
-    const int N = T.n_crystals;
-    const long long total = (long long)T.n_holes0 * N * N;
-    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < n_words;
-         w += (long long)gridDim.x * blockDim.x) {
-        const long long bit0 = w * 32;
-        int i = (int)(bit0 / ((long long)N * N));
-        long long rem = bit0 - (long long)i * N * N;
-        int j = (int)(rem / N);
-        int k = (int)(rem - (long long)j * N);
-        uint32_t word = 0u;
-        for (int b = 0; b < 32 && bit0 + b < total; ++b) {
-            if (collimator_bit(T.crystal_raw, T.hole_raw, i, j, k)) word |= 1u << b;
-            if (++k == N) {
-                k = 0;
-                if (++j == N) {
-                    j = 0;
-                    ++i;
-                }
-            }
+// The line between crystal (or hole) a and crystal b as the bitmaps' cone tests see it.
+struct PairAxis {
+    float4 a, b;
+    float ux, uy, uz;            // unit vector a -> b
+    float ca, cb;                // R_b / |ab|, R_a / |ab|
+};
+
+__device__ __forceinline__ PairAxis pair_axis(const float4& a, const float4& b) {
+    PairAxis p;
+    p.a = a;
+    p.b = b;
+    p.ux = b.x - a.x;
+    p.uy = b.y - a.y;
+    p.uz = b.z - a.z;
+    const float inv = rsqrtf(fmaf(p.ux, p.ux, fmaf(p.uy, p.uy, p.uz * p.uz)));
+    p.ux *= inv;
+    p.uy *= inv;
+    p.uz *= inv;
+    p.ca = b.w * inv;
+    p.cb = a.w * inv;
+    return p;
+}
+
+// The bitmap's bit of (i, j, k), i < j crystals or i hole, j crystal; p = pair_axis of i and j.
+template <int KIND>
+__device__ __forceinline__ bool pair_bit(const ScatterTables& T, const PairAxis& p, int i, int j, int k) {
+    const float4 c = T.crystal_raw[k];
+    int f = cone_quick(c, p.a.x, p.a.y, p.a.z, p.ux, p.uy, p.uz, p.ca);                   // seen from i
+    if (KIND == kScatterCrystal) {
+        if (f != 1) {
+            const int g = cone_quick(c, p.b.x, p.b.y, p.b.z, -p.ux, -p.uy, -p.uz, p.cb);   // seen from j
+            f = g == 1 ? 1 : (f | g);                                                     // -1 when either is unclear
         }
-        words[w] = word;
+        return f < 0 ? crystal_bit(T.crystal_raw, i, j, k) : f == 1;
+    }
+    return f < 0 ? collimator_bit(T.crystal_raw, T.hole_raw, i, j, k) : f == 1;
+}
+
+// Bitmap words: lane = bit, so a warp's loads of the crystals k are consecutive; each
+// lane keeps the word of its own turn and 32 words are stored together.  A bit is
+// decided by cone_quick and, when that cannot call, by the reference's expression
+// (about 500 instructions: every bit took it before, 59.5 ms for 2048 crystals).
+// Crystal pairs: bit = (i N - i (i + 1) / 2 + j) N + k, i <= j; set for i < j, k != i, j.
+// Collimator: bit = i N^2 + j N + k for layer-0 hole i, crystals j, k.
+template <int KIND>
+__global__ void __launch_bounds__(256) bitmap_kernel(uint32_t* __restrict__ words, long long n_words, ScatterTables T) {
+    const int N = T.n_crystals, lane = threadIdx.x & 31;
+    const long long total = KIND == kScatterCrystal ? ((long long)N * (N + 1) / 2) * N : (long long)T.n_holes0 * N * N;
+    const long long n_groups = (n_words + 31) / 32;
+    long long pair = -1;
+    int i = 0, j = 0;
+    PairAxis axis{};
+    for (long long g = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; g < n_groups;
+         g += ((long long)gridDim.x * blockDim.x) >> 5) {
+        long long next = g * 1024 + lane;              // this lane's bit of the group's first word
+        long long at = next / N;
+        int k = (int)(next - at * N);
+        uint32_t mine = 0u;
+        for (int w = 0; w < 32; ++w, next += 32, k += 32) {
+            while (k >= N) {
+                k -= N;
+                ++at;
+            }
+            bool set = false;
+            if (next < total) {
+                if (at != pair) {
+                    pair = at;
+                    if (KIND == kScatterCrystal) {
+                        i = pair_row(pair, N);
+                        j = (int)(pair - ((long long)i * N - (long long)i * (i - 1) / 2)) + i;
+                    } else {
+                        i = (int)(pair / N);
+                        j = (int)(pair - (long long)i * N);
+                    }
+                    axis = pair_axis(KIND == kScatterCrystal ? T.crystal_raw[i] : T.hole_raw[i], T.crystal_raw[j]);
+                }
+                if (KIND != kScatterCrystal || (i < j && k != i && k != j)) set = pair_bit<KIND>(T, axis, i, j, k);
+            }
+            const uint32_t word = __ballot_sync(0xffffffffu, set);
+            if (w == lane) mine = word;
+        }
+        if (g * 32 + lane < n_words) words[g * 32 + lane] = mine;
     }
 }
 
@@ -135,16 +181,36 @@ __global__ void bitmap_collimator_kernel(uint32_t* words, long long n_words, Sca
 // crystal before its unit (:1371-1382), and the absorption chord (:1385-1392).
 // The detector unit is the whole crystal (the reference's divide = 1), whose
 // centre is the crystal centre.
+// A warp takes 32 neighbouring detectors and one scatter point S.  The crystals their
+// segments can meet are those whose box meets the hull of S and the detectors' box B, the
+// union of the boxes S + l (B - S), l in [0, 1]: every face gives a bound on l, and the
+// test is whether the bounds leave any (lane = crystal, 32 at a time, boxes grown by
+// 0.01 mm).  The survivors, some dozens of thousands, are walked by all lanes, each with
+// its own segment: chord_quick drops the uncrossed ones, crossed ones take
+// chord_through's value if the bitmap flags them - read from a given bitmap, or decided
+// here for the crossed crystal alone, without building the N^3 / 2 bits (walking the
+// flagged crystals of a computed bitmap took 24.7 ms for 2048 x 2048 pairs).
 template <int KIND>
-__global__ void scatter_pair_kernel(DevGeometry G, ScatterTables T, const uint32_t* __restrict__ bitmap,
-                                    const int* __restrict__ perm, int r0, int r1, float4* __restrict__ pair,
-                                    int n_sources) {
+__global__ void __launch_bounds__(128) scatter_pair_kernel(const __grid_constant__ DevGeometry G,
+                                                           const __grid_constant__ ScatterTables T,
+                                                           const uint32_t* __restrict__ bitmap,
+                                                           const int* __restrict__ perm, int r0, int r1,
+                                                           float4* __restrict__ pair, int n_sources) {
     const int N = T.n_crystals;
     const int r = r0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= r1) return;
-    const int d = perm[r];
+    const int d = perm[min(r, r1 - 1)];
     const long long ld = r1 - r0;
     const float4 Dp = G.c.pos[d], Dsz = G.c.size[d], Dr = G.c.rot[d];
+    const int lane = threadIdx.x & 31;
+    Box3 B{Dp.x, Dp.y, Dp.z, Dp.x, Dp.y, Dp.z};          // of the warp's detector centres
+    for (int o = 16; o > 0; o >>= 1) {
+        B.x1 = fminf(B.x1, __shfl_xor_sync(0xffffffffu, B.x1, o));
+        B.y1 = fminf(B.y1, __shfl_xor_sync(0xffffffffu, B.y1, o));
+        B.z1 = fminf(B.z1, __shfl_xor_sync(0xffffffffu, B.z1, o));
+        B.x2 = fmaxf(B.x2, __shfl_xor_sync(0xffffffffu, B.x2, o));
+        B.y2 = fmaxf(B.y2, __shfl_xor_sync(0xffffffffu, B.y2, o));
+        B.z2 = fmaxf(B.z2, __shfl_xor_sync(0xffffffffu, B.z2, o));
+    }
     for (int q = blockIdx.y; q < n_sources; q += gridDim.y) {
         float4 S;
         int s;
@@ -155,43 +221,97 @@ __global__ void scatter_pair_kernel(DevGeometry G, ScatterTables T, const uint32
             S = T.hole_src[q];
             s = q;
         }
-        float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (!(KIND == kScatterCrystal && s == d)) {
-            float a_pe = 0.0f, a_c = 0.0f;
-            long long base;
+        const bool on = r < r1 && !(KIND == kScatterCrystal && s == d);
+        long long base;
+        if (KIND == kScatterCrystal) {
+            const int lo = s < d ? s : d, hi = s < d ? d : s;
+            base = ((long long)lo * N - (long long)lo * (lo + 1) / 2 + hi) * N;
+        } else {
+            base = ((long long)s * N + d) * N;
+        }
+        const float dx = Dp.x - S.x, dy = Dp.y - S.y, dz = Dp.z - S.z;
+        const float len2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), inv_len = rsqrtf(len2);
+        ChordRay cr = make_chord_ray(S.x, S.y, S.z, dx, dy, dz, len2 * inv_len, T.chord_delta);
+        const bool flat = !cr.ok && flatten(&cr, dx, dy, dz);   // source and detector in one layer, row or column
+        PairAxis axis{};
+        int pi = s, pj = d;
+        if (!bitmap) {
             if (KIND == kScatterCrystal) {
-                const int lo = s < d ? s : d, hi = s < d ? d : s;
-                base = ((long long)lo * N - (long long)lo * (lo + 1) / 2 + hi) * N;
-            } else {
-                base = ((long long)s * N + d) * N;
+                pi = min(s, d);
+                pj = max(s, d);
             }
-            const long long w_end = (base + N - 1) >> 5;
-            for (long long wi = base >> 5; wi <= w_end; ++wi) {
-                uint32_t bits = __ldg(bitmap + wi);
-                const long long first = wi << 5;
-                if (first < base) bits &= ~0u << (int)(base - first);
-                if (first + 31 > base + N - 1) {
-                    const int keep = (int)(base + N - first);
-                    bits &= keep >= 32 ? ~0u : ((1u << keep) - 1u);
+            axis = pair_axis(KIND == kScatterCrystal ? T.crystal_raw[pi] : T.hole_raw[pi], T.crystal_raw[pj]);
+        }
+        // bounds on l: l * face >= gap (face > 0: from below, < 0: from above)
+        const float face[6] = {B.x2 - S.x, B.y2 - S.y, B.z2 - S.z, S.x - B.x1, S.y - B.y1, S.z - B.z1};
+        float inv_face[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) inv_face[a] = fabsf(face[a]) > 1e-4f ? __fdividef(1.0f, face[a]) : 0.0f;
+        float a_pe = 0.0f, a_c = 0.0f;
+        for (int k0 = 0; k0 < N; k0 += 32) {
+            bool meets = false;
+            if (k0 + lane < N) {
+                const float4 lo = __ldg(G.c.lo + k0 + lane), hi = __ldg(G.c.hi + k0 + lane);
+                const float m = 0.01f;
+                const float gap[6] = {lo.x - m - S.x, lo.y - m - S.y, lo.z - m - S.z, S.x - hi.x - m, S.y - hi.y - m, S.z - hi.z - m};
+                float from = 0.0f, to = 1.0f;
+                bool empty = false;
+#pragma unroll
+                for (int a = 0; a < 6; ++a) {
+                    const float l = gap[a] * inv_face[a];
+                    if (face[a] > 1e-4f) from = fmaxf(from, l);
+                    else if (face[a] < -1e-4f) to = fminf(to, l);
+                    else empty |= gap[a] > 1e-4f;
                 }
-                while (bits) {
-                    const int b = __ffs(bits) - 1;
-                    bits &= bits - 1u;
-                    const int k = (int)(first + b - base);
-                    if (k == d || (KIND == kScatterCrystal && k == s)) continue;
-                    const float4 kp = G.c.pos[k], ks = G.c.size[k], kr = G.c.rot[k], kph = G.c.phys[k];
-                    const float xa = (S.x - kp.x) * kr.x - (S.z - kp.z) * kr.y;
-                    const float ya = S.y - kp.y;
-                    const float za = (S.x - kp.x) * kr.y + (S.z - kp.z) * kr.x;
-                    const float xb = (Dp.x - kp.x) * kr.x - (Dp.z - kp.z) * kr.y;
-                    const float yb = Dp.y - kp.y;
-                    const float zb = (Dp.x - kp.x) * kr.y + (Dp.z - kp.z) * kr.x;
-                    const Box3 kb{-0.5f * ks.x, -0.5f * ks.y, -0.5f * ks.z, 0.5f * ks.x, 0.5f * ks.y, 0.5f * ks.z};
-                    const float len = chord_through(xa, ya, za, xb, yb, zb, kb);
-                    a_pe += len * kph.x;
-                    a_c += len * kph.y;
-                }
+                meets = !empty && from <= to;
             }
+            uint32_t any = __ballot_sync(0xffffffffu, meets);
+            if (!any) continue;
+            // which of them this lane's pair counts
+            uint32_t bits = on ? 0xffffffffu : 0u;
+            if (on && bitmap) {
+                const long long bit = base + k0, w = bit >> 5;
+                const int sh = (int)(bit & 31);
+                const uint32_t lo = __ldg(bitmap + w), hi = sh && (w << 5) + 32 < base + N ? __ldg(bitmap + w + 1) : 0u;
+                bits = __funnelshift_r(lo, hi, sh);
+            }
+            if ((d & ~31) == k0) bits &= ~(1u << (d & 31));
+            if (KIND == kScatterCrystal && (s & ~31) == k0) bits &= ~(1u << (s & 31));
+            while (any) {
+                const int b = __ffs(any) - 1, k = k0 + b;
+                any &= any - 1u;
+                const float4 kp = __ldg(G.c.pos + k), ks = __ldg(G.c.size + k), kr = __ldg(G.c.rot + k);
+                if (!(bits >> b & 1u)) continue;
+                const float hx = 0.5f * ks.x, hy = 0.5f * ks.y, hz = 0.5f * ks.z;
+                const float xa = (S.x - kp.x) * kr.x - (S.z - kp.z) * kr.y;
+                const float ya = S.y - kp.y;
+                const float za = (S.x - kp.x) * kr.y + (S.z - kp.z) * kr.x;
+                const float xb = (Dp.x - kp.x) * kr.x - (Dp.z - kp.z) * kr.y;
+                const float yb = Dp.y - kp.y;
+                const float zb = (Dp.x - kp.x) * kr.y + (Dp.z - kp.z) * kr.x;
+                ChordRay c = cr;
+                c.px = xa;
+                c.py = ya;
+                c.pz = za;
+                if (kr.x != 1.0f || kr.y != 0.0f)
+                    c = make_chord_ray(xa, ya, za, fmaf(dx, kr.x, -dz * kr.y), dy, fmaf(dx, kr.y, dz * kr.x), cr.len,
+                                       2.0f * T.chord_delta);
+                float chord;
+                int f = -1;
+                if (c.ok && cr.ok) f = chord_quick(c, 0.0f, 0.0f, 0.0f, hx, hy, hz, &chord);
+                else if (flat && kr.x == 1.0f && kr.y == 0.0f)
+                    f = chord_filter(c, 0.0f, 0.0f, 0.0f, hx, hy, hz, T.chord_delta, &chord) == 0 ? 0 : -1;
+                if (f == 0) continue;
+                const float len = f > 0 ? chord_value(xa, ya, za, xb, yb, zb, hx, hy, hz, c.ix, c.iy, c.iz, inv_len)
+                                        : chord_through(xa, ya, za, xb, yb, zb, Box3{-hx, -hy, -hz, hx, hy, hz});
+                if (len == 0.0f || (!bitmap && !pair_bit<KIND>(T, axis, pi, pj, k))) continue;
+                const float4 kph = __ldg(G.c.phys + k);
+                a_pe += len * kph.x;
+                a_c += len * kph.y;
+            }
+        }
+        float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (on) {
             // scatter point in the detecting crystal's frame
             const float xs = (S.x - Dp.x) * Dr.x - (S.z - Dp.z) * Dr.y;
             const float ys = S.y - Dp.y;
@@ -207,7 +327,7 @@ __global__ void scatter_pair_kernel(DevGeometry G, ScatterTables T, const uint32
             const float labs = chord_through(xs, ys, zs, xt, yt, zt, ub);
             out = make_float4(a_pe, a_c, l1 - l2, labs);
         }
-        pair[(long long)q * ld + (r - r0)] = out;
+        if (r < r1) pair[(long long)q * ld + (r - r0)] = out;
     }
 }
 
@@ -769,15 +889,15 @@ int64_t collimator_bitmap_words(int n, int h0) {
 
 cudaError_t launch_bitmap_crystal(uint32_t* words, int64_t n_words, const ScatterTables& T, cudaStream_t s) {
     if (n_words <= 0) return cudaSuccess;
-    const long long blocks = std::min<long long>((n_words + 255) / 256, 148LL * 64);
-    bitmap_crystal_kernel<<<(unsigned)blocks, 256, 0, s>>>(words, n_words, T);
+    const long long blocks = std::min<long long>((n_words + 255) / 256, 148LL * 64);   // a warp per 32 words
+    bitmap_kernel<kScatterCrystal><<<(unsigned)blocks, 256, 0, s>>>(words, n_words, T);
     return cudaGetLastError();
 }
 
 cudaError_t launch_bitmap_collimator(uint32_t* words, int64_t n_words, const ScatterTables& T, cudaStream_t s) {
     if (n_words <= 0) return cudaSuccess;
     const long long blocks = std::min<long long>((n_words + 255) / 256, 148LL * 64);
-    bitmap_collimator_kernel<<<(unsigned)blocks, 256, 0, s>>>(words, n_words, T);
+    bitmap_kernel<kScatterCollimator><<<(unsigned)blocks, 256, 0, s>>>(words, n_words, T);
     return cudaGetLastError();
 }
 

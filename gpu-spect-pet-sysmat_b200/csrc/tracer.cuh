@@ -254,6 +254,26 @@ SM_HD ChordRay make_chord_ray(float px, float py, float pz, float dx, float dy, 
     return c;
 }
 
+// A segment with one axis below the reference's degenerate extent, which it leaves out
+// of the slabs: there the segment stays inside the slab or misses the box.  Makes r fit
+// for chord_filter's "no chord" call (a steep reciprocal says the same); false when an
+// axis is too near the limit to tell, or two are below it (the reference then counts a
+// segment that starts on the box too).
+SM_HD bool flatten(ChordRay* r, float dx, float dy, float dz) {
+    const float d[3] = {fabsf(dx), fabsf(dy), fabsf(dz)};
+    float* inv[3] = {&r->ix, &r->iy, &r->iz};
+    float* mag[3] = {&r->ax, &r->ay, &r->az};
+    int flat = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (d[a] < 0.0009f) {
+            *inv[a] = *mag[a] = 1e9f;
+            ++flat;
+        } else if (!(d[a] > 0.002f)) return false;
+    }
+    return flat == 1;
+}
+
 // chord_through of the box of half sizes (hx, hy, hz) about (cx, cy, cz), when
 // the answer is clear: 1 (the chord, in `chord`), 0 (no chord) or -1 (too
 // close to call: chord_through decides).  In units of the segment, axis i of

@@ -2,7 +2,7 @@
 // chord_through and chord_hole on the host: chord_filter_check SEED COUNT RANGE.
 // Prints "<wrong calls> <clear hits> <clear misses> <unclear> <largest value error>
 // <holes called missed> <holes called crossed> <of them with another value>
-// <crossed boxes with another chord_value>".
+// <crossed boxes with another chord_value> <flattened segments>".
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -20,7 +20,7 @@ int main(int argc, char** argv) {
     auto U = [&](float a, float b) { return std::uniform_real_distribution<float>(a, b)(gen); };
     auto side = [&](float h) { return U(0, 1) < 0.5f ? -h : h; };
     const float lat = 0.35f * range;   // image and detector half width; depth up to half the range
-    long wrong = 0, hits = 0, misses = 0, unclear = 0, hole_misses = 0, hole_hits = 0, hole_other = 0, other = 0;
+    long wrong = 0, hits = 0, misses = 0, unclear = 0, hole_misses = 0, hole_hits = 0, hole_other = 0, other = 0, flat = 0;
     double worst = 0.0;
     for (long i = 0; i < n; ++i) {
         const float hx = U(0.3f, 2), hy = U(0.3f, 4), hz = U(0.3f, 2), near = 3 * delta;
@@ -48,6 +48,9 @@ int main(int argc, char** argv) {
             py = ky - hy + U(-0.003f, 0.003f);
             pz = kz + U(-1, 1) * hz;
         }
+        if (i % 17 == 0) qx = px + U(-0.003f, 0.003f);       // below the degenerate extent, or nearly
+        if (i % 34 == 0) qz = pz;
+        if (i % 51 == 0) qy = py;
         const float dx = qx - px, dy = qy - py, dz = qz - pz, len = std::sqrt(dx * dx + dy * dy + dz * dz);
         const ChordRay r = make_chord_ray(px, py, pz, dx, dy, dz, len, delta);
         const Box3 box{-hx, -hy, -hz, hx, hy, hz};
@@ -69,6 +72,12 @@ int main(int argc, char** argv) {
                                 (qx - kx) * s + (qz - kz) * c, hx, hy, hz, k.ix, k.iy, k.iz, 1 / len);
             ref = chord_through(ax * c - az * s, py - ky, ax * s + az * c, (qx - kx) * c - (qz - kz) * s, qy - ky,
                                 (qx - kx) * s + (qz - kz) * c, box);
+        }
+        ChordRay e = r;
+        if (i % 3 && !r.ok && flatten(&e, dx, dy, dz)) {
+            float c;
+            wrong += chord_filter(e, kx, ky, kz, hx, hy, hz, delta, &c) == 0 && ref != 0;
+            ++flat;
         }
         if (fq >= 0) wrong += (fq != 0) != (ref != 0) || (f >= 0 && f != fq) || (fq == 1 && f == 1 && quick != chord);
         if (f < 0) ++unclear;
@@ -97,6 +106,6 @@ int main(int argc, char** argv) {
             wrong += (hf == 0 && hr != 0) || (hf == 1 && (hr == 0 || std::fabs(hc - hr) > 2e-6f * len));
         }
     }
-    std::printf("%ld %ld %ld %ld %.3g %ld %ld %ld %ld\n", wrong, hits, misses, unclear, worst, hole_misses, hole_hits, hole_other, other);
+    std::printf("%ld %ld %ld %ld %.3g %ld %ld %ld %ld %ld\n", wrong, hits, misses, unclear, worst, hole_misses, hole_hits, hole_other, other, flat);
     return 0;
 }

@@ -28,7 +28,7 @@ def test_clear_calls_are_the_exact_ones(check, coordinate_range):
     assert hits > 100000 and misses > 100000
     assert unclear < 0.35 * (hits + misses)      # every second ray aims at an edge
     assert float(out[4]) <= 2.0
-    hole_misses, hole_hits, hole_other, other = map(int, out[5:])
+    hole_misses, hole_hits, hole_other, other, flat = map(int, out[5:])
     assert hole_misses > 50000 and hole_hits > 50000        # three holes in five have their wall near the ray
-    assert other < 1e-2 * hits
+    assert other < 1e-2 * hits and flat > 10000
     assert hole_other < 1e-3 * hole_hits                    # the exact form's value but for rare last bits
