@@ -290,9 +290,10 @@ int sm_scatter_legacy(int parts, float* parameter_Collimator, float* parameter_D
  * accumulators in tensor memory) on device buffers of the current device:
  *   C[i][j] = s_i * sum_k A[i][k] B[j][k] (+ bias[j]) (+ C[i][j] if accumulate)
  * with A[i][k] = a[i * a_ms + k * a_ks], B[j][k] = b[j * b_ns + k * b_ks]
- * (bf16, any strides; k-contiguous operands load fastest), C fp32 row-major
- * with pitch ldc, s_i = row_scale[i] or alpha.  n_tile (64 / 128 / 256) is
- * the column width per CTA.  error (device int, may be NULL) is set to 1 if
+ * (bf16, any strides; k-contiguous operands with 16-byte aligned base and
+ * pitch load fastest), C fp32 row-major
+ * with pitch ldc, s_i = row_scale[i] or alpha.  n_tile must be 64, 128 or 256;
+ * the launch picks its own tile width (results do not depend on it).  error (device int, may be NULL) is set to 1 if
  * the kernel's bounded wait on its own MMAs ran out.  Asynchronous on stream. */
 int sm_gemm_bf16(int m, int n, int k, const void* a, int64_t a_ms, int64_t a_ks, const void* b, int64_t b_ns,
                  int64_t b_ks, float* c, int64_t ldc, float alpha, const float* row_scale, const float* bias,
