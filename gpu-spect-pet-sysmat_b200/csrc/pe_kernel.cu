@@ -199,10 +199,10 @@ __device__ __forceinline__ int cone_filter(const ConeSelf& cs, const Vec3& p, fl
                                            float crit_scaled) {
     float dx = xk - p.x, dy = yk - p.y, dz = zk - p.z;
     float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    float inv = rsqrtf(d2);
+    float inv = fast_rsqrt(d2);
     float ex = fmaf(dx, inv, -cs.ux), ey = fmaf(dy, inv, -cs.uy), ez = fmaf(dz, inv, -cs.uz);
     const float e2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-    const float lhs = e2 > 0.0f ? e2 * rsqrtf(e2) : 0.0f;   // within 1e-6 relative of sqrt(e2)
+    const float lhs = e2 > 1e-30f ? e2 * fast_rsqrt(e2) : 0.0f;   // within 1e-6 relative of sqrt(e2)
     float rhs = fmaf(crit_scaled, inv, cs.crit_self);
     float diff = lhs - rhs;
     if (diff < -kConeMargin) return 1;
@@ -220,7 +220,7 @@ __device__ __forceinline__ bool cone_sure(const Vec3& p0, float rho, float kx, f
                                           float dy, float dz, float rd) {
     const float ax = kx - p0.x, ay = ky - p0.y, az = kz - p0.z, bx = dx - p0.x, by = dy - p0.y, bz = dz - p0.z;
     const float a2 = fmaf(ax, ax, fmaf(ay, ay, az * az)), b2 = fmaf(bx, bx, fmaf(by, by, bz * bz));
-    const float ia = rsqrtf(a2), ib = rsqrtf(b2), da = a2 * ia, db = b2 * ib;
+    const float ia = fast_rsqrt(a2), ib = fast_rsqrt(b2), da = a2 * ia, db = b2 * ib;
     const float m = fminf(da, db) - rho;
     const float ux = fmaf(ax, ia, -bx * ib), uy = fmaf(ay, ia, -by * ib), uz = fmaf(az, ia, -bz * ib);
     const float lhs = sqrtf(fmaf(ux, ux, fmaf(uy, uy, uz * uz)));
@@ -254,8 +254,8 @@ __device__ __forceinline__ Bundle make_bundle(const Box3& A, const Box3& B) {
     b.A = A;
     b.B = B;
     b.ordered = A.y2 < B.y1;
-    b.inv2 = __fdividef(1.0f, B.y2 - A.y2);
-    b.inv1 = __fdividef(1.0f, B.y1 - A.y1);
+    b.inv2 = fast_rcp(B.y2 - A.y2);
+    b.inv1 = fast_rcp(B.y1 - A.y1);
     return b;
 }
 
@@ -446,7 +446,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
 
     const float dxw = q.x - p.x, dy = q.y - p.y, dzw = q.z - p.z;
     const float dsq = fmaf(dy, dy, fmaf(dxw, dxw, dzw * dzw));
-    const float inv_r = rsqrtf(dsq);
+    const float inv_r = fast_rsqrt(dsq);
     const float r = dsq * inv_r;
     const ChordRay cr = make_chord_ray(p.x, p.y, p.z, dxw, dy, dzw, r, P.chord_delta);
 
@@ -590,7 +590,7 @@ __device__ __forceinline__ float trace_ray_global(const DevGeometry& G, const De
     seg.ordered = p.y < q.y;
     const float dxw = q.x - p.x, dy = q.y - p.y, dzw = q.z - p.z;
     const float dsq = fmaf(dy, dy, fmaf(dxw, dxw, dzw * dzw));
-    const float inv_r = rsqrtf(dsq);
+    const float inv_r = fast_rsqrt(dsq);
     const float r = dsq * inv_r;
     const ChordRay cr = make_chord_ray(p.x, p.y, p.z, dxw, dy, dzw, r, 0.0f);
     seg.inv_dy = fast_rcp(dy);
@@ -1060,7 +1060,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                     const int gn = min(P.group, n_pts - g0);
                     const int g1 = gn == P.group ? n_pts - n_pts % P.group : n_pts;
                     const int cb = gn * P.dY;                  // rays per sub-cell column
-                    const float inv_cb = __fdividef(1.0f, (float)cb);
+                    const float inv_cb = fast_rcp((float)cb);
                     const int nr = gn * P.n_sc;
                     for (int q0 = 0; q0 < nr; q0 += 32) {
                         const int e = q0 + lane;

@@ -83,7 +83,7 @@ __device__ __forceinline__ int pair_row(long long pair, int N) {
 __device__ __forceinline__ int cone_quick(const float4& k, float ax, float ay, float az, float ux, float uy, float uz,
                                           float c) {
     const float dx = k.x - ax, dy = k.y - ay, dz = k.z - az;
-    const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+    const float inv = fast_rsqrt(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
     const float cosine = fmaf(dx, ux, fmaf(dy, uy, dz * uz)) * inv;
     const float rhs = fmaf(k.w, inv, c), r2 = rhs * rhs;
     const float diff = fmaf(-2.0f, cosine, 2.0f) - r2, band = fmaf(1e-4f, r2, 1e-5f);
@@ -104,7 +104,7 @@ __device__ __forceinline__ PairAxis pair_axis(const float4& a, const float4& b) 
     p.ux = b.x - a.x;
     p.uy = b.y - a.y;
     p.uz = b.z - a.z;
-    const float inv = rsqrtf(fmaf(p.ux, p.ux, fmaf(p.uy, p.uy, p.uz * p.uz)));
+    const float inv = fast_rsqrt(fmaf(p.ux, p.ux, fmaf(p.uy, p.uy, p.uz * p.uz)));
     p.ux *= inv;
     p.uy *= inv;
     p.uz *= inv;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(128) scatter_pair_kernel(const __grid_constant
             base = ((long long)s * N + d) * N;
         }
         const float dx = Dp.x - S.x, dy = Dp.y - S.y, dz = Dp.z - S.z;
-        const float len2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), inv_len = rsqrtf(len2);
+        const float len2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), inv_len = fast_rsqrt(len2);
         ChordRay cr = make_chord_ray(S.x, S.y, S.z, dx, dy, dz, len2 * inv_len, T.chord_delta);
         const bool flat = !cr.ok && flatten(&cr, dx, dy, dz);   // source and detector in one layer, row or column
         PairAxis axis{};
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(128) scatter_pair_kernel(const __grid_constant
         const float face[6] = {B.x2 - S.x, B.y2 - S.y, B.z2 - S.z, S.x - B.x1, S.y - B.y1, S.z - B.z1};
         float inv_face[6];
 #pragma unroll
-        for (int a = 0; a < 6; ++a) inv_face[a] = fabsf(face[a]) > 1e-4f ? __fdividef(1.0f, face[a]) : 0.0f;
+        for (int a = 0; a < 6; ++a) inv_face[a] = fabsf(face[a]) > 1e-4f ? fast_rcp(face[a]) : 0.0f;
         float a_pe = 0.0f, a_c = 0.0f;
         for (int k0 = 0; k0 < N; k0 += 32) {
             bool meets = false;
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
             }
             todo = __any_sync(0xffffffffu, live) ? S.todo[k][col] & mine : 0u;
             ax = pt.x - I.x; ay = pt.y - I.y; az = pt.z - I.z;
-            inv_a = rsqrtf(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+            inv_a = fast_rsqrt(fmaf(ax, ax, fmaf(ay, ay, az * az)));
         };
         open_point();
         for (;;) {

@@ -14,26 +14,22 @@ namespace smb {
 constexpr float kDelta = 0.01f;   // the reference's DeltaTheta, as a float
 constexpr float kNodesPerRad = (float)kKnNodes / 3.14159265358979323846f;
 
-SM_HD float sm_rsqrt(float x) {
-#ifdef __CUDA_ARCH__
-    return rsqrtf(x);
-#else
-    return 1.0f / std::sqrt(x);
-#endif
-}
+// Fast quotient, root and reciprocal root for values (never for a decision the
+// reference takes): about 2 ulp, against ~10 instructions for the IEEE forms this
+// translation unit is compiled with.
+SM_HD float sm_rsqrt(float x) { return fast_rsqrt(x); }
 
-// Fast quotient and square root for values (never for a decision the
-// reference takes): about 2 ulp, against ~10 instructions for the IEEE forms
-// this translation unit is compiled with.
 SM_HD float sm_fdiv(float a, float b) {
 #ifdef __CUDA_ARCH__
-    return __fdividef(a, b);
+    float r;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 #else
     return a / b;
 #endif
 }
 
-SM_HD float sm_fsqrt(float x) { return x > 0.0f ? x * sm_rsqrt(x) : 0.0f; }
+SM_HD float sm_fsqrt(float x) { return x > 1e-37f ? x * sm_rsqrt(x) : 0.0f; }
 
 SM_HD int sm_rint(float x) {
 #ifdef __CUDA_ARCH__

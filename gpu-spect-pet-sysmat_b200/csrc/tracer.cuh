@@ -29,6 +29,30 @@ struct Box3 {
     float x1, y1, z1, x2, y2, z2;
 };
 
+// The hardware's approximate reciprocal and reciprocal square root.  Subnormal operands
+// count as zero: nothing here divides by or takes the root of one (lengths are at least a
+// rounding of the coordinates, or exactly zero), and the forms that keep subnormals spend
+// three more instructions on rescaling.
+SM_HD float fast_rcp(float d) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return r;
+#else
+    return 1.0f / d;
+#endif
+}
+
+SM_HD float fast_rsqrt(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.0f / std::sqrt(x);
+#endif
+}
+
 // Entry/exit parameters of one slab for a segment parameterised by length
 // t_total (PESysMatGen.cu:57-64 and every slab of :19-151).
 SM_HD void slab_pair(float a_in, float a_out, float lo, float hi, float t_total, float& t_lo,
@@ -227,14 +251,6 @@ struct ChordRay {
     bool ok;        // no axis is near the reference's degenerate extent (0.001)
 };
 
-SM_HD float fast_rcp(float d) {
-#ifdef __CUDA_ARCH__
-    return __fdividef(1.0f, d);
-#else
-    return 1.0f / d;
-#endif
-}
-
 // 1 / d to about one unit in the last place.
 SM_HD float chord_rcp(float d) {
     const float r = fast_rcp(d);
@@ -330,13 +346,7 @@ SM_HD float near_root(float x, float r) {   // r ~ 1 / sqrt(x)
     return fmaf(fmaf(-s, s, x), 0.5f * r, s);
 }
 
-SM_HD float near_sqrt(float x) {
-#ifdef __CUDA_ARCH__
-    return near_root(x, rsqrtf(x));
-#else
-    return near_root(x, 1.0f / std::sqrt(x));
-#endif
-}
+SM_HD float near_sqrt(float x) { return near_root(x, fast_rsqrt(x)); }
 
 // chord_through's own value, operation for operation, for a segment a -> b that a
 // filter called a clear chord of the box of half sizes h about the origin; ix, iy,
