@@ -166,9 +166,10 @@ __device__ __forceinline__ ConeSelf cone_self(const Detecting& D, const Vec3& p)
     return c;
 }
 
-// The group's table when there is one, else computed for this ray (few rays need it then: see kConeSure).
+// From the group's table (TABLE), else computed for this ray (few rays need it then: see kConeSure).
+template <bool TABLE>
 __device__ __forceinline__ ConeSelf cone_of(const float4* table, const Detecting& D, const Vec3& p) {
-    if (!table) return cone_self(D, p);
+    if (!TABLE) return cone_self(D, p);
     const float4 c = *table;
     return ConeSelf{c.x, c.y, c.z, c.w};
 }
@@ -426,6 +427,11 @@ __device__ __forceinline__ SubCell sub_cell(const Detecting& D, const PeSmem& S,
     return c;
 }
 
+// Work counters of a warp (sm_pe_set_counters).
+struct RayCounts {
+    unsigned long long rays, crystal, hole, cone;
+};
+
 // One ray: sub-point p (world) and ps (detecting crystal frame), sub-cell
 // `cell`.  pass_c / pass_h: the candidates the warp pass's bundle of rays
 // can reach (a superset of those this ray can reach).  The reference counts a
@@ -434,13 +440,12 @@ __device__ __forceinline__ SubCell sub_cell(const Detecting& D, const PeSmem& S,
 // either way, so the cone test (`csp`: the sub-point's ConeSelf) is taken only
 // for candidates with a nonzero chord.  Returns the contribution; in RECORD
 // mode also the hit record.
-template <bool RECORD, bool FEW>
+template <bool RECORD, bool FEW, bool COUNT>
 __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry& G, const PeSmem& S,
                                            const WarpLists& L, unsigned plates_sure, bool any_hole,
                                            const float4* csp, const Detecting& D, const Vec3& p,
                                            const Vec3& ps, const SubCell& cell, int* rec, int* status,
-                                           unsigned long long* n_cry, unsigned long long* n_hole,
-                                           unsigned long long* n_cone) {
+                                           RayCounts& n) {
     const float xDs = cell.xDs, yDs = cell.yDs, zDs = cell.zDs;
     const Vec3 q = cell.q;
 
@@ -476,15 +481,15 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
                 int f = -1;
                 if (dy > 0.0f && p.y < ha.y)
                     f = hole_filter(p.x, p.y, p.z, dxw, dy, dzw, cr.iy, r, ha.x, ha.y, ha.z, ha.w, hbv.x, P.chord_delta, &len);
-                if (n_hole && f) ++*n_hole;
+                if (COUNT && f) ++n.hole;
                 if (f < 0) {
                     len = hole_chord_exact(p, q, ha, hbv.x);
                     f = len != 0.0f;
                 }
                 if (!f) continue;
                 if (!(e & kConeSure)) {
-                    if (n_cone) ++*n_cone;
-                    const ConeSelf cs = cone_of(csp, D, p);
+                    if (COUNT) ++n.cone;
+                    const ConeSelf cs = cone_of<FEW>(csp, D, p);
                     int g = cone_filter(cs, p, ha.x, hbv.w, ha.w, hbv.z);
                     if (g < 0) g = cone_hole_exact(cs, p, ha.x, hbv.w, ha.w, hbv.z) ? 1 : 0;
                     if (!g) continue;
@@ -531,7 +536,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
                 if (f < 0 && kr.ok)
                     f = chord_filter(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, 2.0f * P.chord_delta, &len);
             }
-            if (n_cry && f) ++*n_cry;
+            if (COUNT && f) ++n.crystal;
             if (f < 0 || !cr.ok) {
                 len = crystal_chord_exact(p, q, kp, kh, kc, ks);
                 f = len != 0.0f;
@@ -549,8 +554,8 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
                                       bx * ks + bz * kc, kh.x, kh.y, kh.z, kix, cr.iy, kiz, inv_r);
             }
             if (!(e & kConeSure)) {
-                if (n_cone) ++*n_cone;
-                const ConeSelf cs = cone_of(csp, D, p);
+                if (COUNT) ++n.cone;
+                const ConeSelf cs = cone_of<FEW>(csp, D, p);
                 int g = cone_filter(cs, p, kp.x, kp.y, kp.z, kh.w);
                 if (g < 0) g = cone_crystal_exact(cs, p, kp.x, kp.y, kp.z, 2.0f * kh.w) ? 1 : 0;
                 if (!g) continue;
@@ -704,7 +709,7 @@ __device__ __forceinline__ int warp_append(bool pass, int value, unsigned short*
 
 // One tile (8 crystals x one voxel brick) of geometry G.  Shared by the
 // one-launch-per-geometry kernel and the persistent batch kernel.
-template <bool RECORD, bool FEW>
+template <bool RECORD, bool FEW, bool COUNT>
 __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G, PeSmem& S, long long tile) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -895,10 +900,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
             }
             __syncwarp();
         }
-        unsigned long long cnt_rays = 0, cnt_cry = 0, cnt_hole = 0, cnt_cone = 0;
-        unsigned long long* pc_cry = P.counters ? &cnt_cry : nullptr;
-        unsigned long long* pc_hole = P.counters ? &cnt_hole : nullptr;
-        unsigned long long* pc_cone = P.counters ? &cnt_cone : nullptr;
+        RayCounts counts{};
         // Entries of few rays go VP neighbouring voxels of the brick to a group
         // (P.pair, up to 8): a pass then traces one sub-cell column from all of
         // them, and the lanes of each voxel are summed apart.
@@ -935,12 +937,12 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                 z = iz0 + zb;
             };
             int ix, iy, iz;
-            vox_of(VP == 1 ? 0 : (lane & 7), ix, iy, iz);
+            vox_of(FEW ? (lane & 7) : 0, ix, iy, iz);
             const bool in = (lane & 7) < VP && vl + (lane & 7) < tv && ix < ix1 && iy < iy1 && iz < iz1;
             const unsigned valid = __ballot_sync(0xffffffffu, in) & 0xffu;
             if (!valid) continue;
             int lox = ix, loy = iy, loz = iz, hix = ix, hiy = iy, hiz = iz;
-            if (VP > 1) {
+            if (FEW) {
                 lox = __reduce_min_sync(0xffffffffu, in ? ix : 1 << 30);
                 loy = __reduce_min_sync(0xffffffffu, in ? iy : 1 << 30);
                 loz = __reduce_min_sync(0xffffffffu, in ? iz : 1 << 30);
@@ -1044,7 +1046,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                 // same candidates.  Every full group deals the same sub-cells to the
                 // same passes, so a pass's sub-cells and candidates serve all of them.
                 const int n_pts = VP * P.n_sv;
-                if (VP > 1) {   // one group: its points once for all passes
+                if (FEW) {   // one group: its points once for all passes
                     if (lane < n_pts) {
                         const int u = fast_div(lane, P.n_sv, P.inv_n_sv);
                         int x, y, z;
@@ -1140,7 +1142,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                         for (int s0 = g0; s0 < g1; s0 += gn) {
                             Vec3 p;
                             const float4* csp = nullptr;
-                            if (VP > 1) {
+                            if (FEW) {
                                 const float4 p4 = L.pt[j];
                                 p = Vec3{p4.x, p4.y, p4.z};
                                 csp = &L.cs[j];
@@ -1148,7 +1150,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                                 active = has && ((valid >> lane_vox) & 1u);
                             }
                             if (active) {
-                                if (VP == 1) p = subpoint_of(P, ix, iy, iz, s0 + j);
+                                if (!FEW) p = subpoint_of(P, ix, iy, iz, s0 + j);
                                 // ... in the detecting crystal's frame
                                 Vec3 ps{p.x - D.cx, p.y - D.cy, p.z - D.cz};
                                 if (D.rotated) ps = Vec3{ps.x * D.cm - ps.z * D.sm, ps.y, ps.x * D.sm + ps.z * D.cm};
@@ -1158,9 +1160,9 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                                     rec = P.rec_out + ((long long)rec_slot * P.n_sv * P.n_sc + (long long)(s0 + j) * P.n_sc + c) *
                                                           kRecWords;
                                 }
-                                const float v = trace_ray<RECORD, FEW>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
-                                                                  P.status, pc_cry, pc_hole, pc_cone);
-                                if (P.counters) ++cnt_rays;
+                                const float v = trace_ray<RECORD, FEW, COUNT>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
+                                                                  P.status, counts);
+                                if (COUNT) ++counts.rays;
                                 // Kahan summation of the lane's rays.
                                 const float y2 = v - comp;
                                 const float t = acc + y2;
@@ -1188,18 +1190,18 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                 }
             }
         }
-        if (P.counters) {
+        if (COUNT) {
             for (int o = 16; o > 0; o >>= 1) {
-                cnt_rays += __shfl_xor_sync(0xffffffffu, cnt_rays, o);
-                cnt_cry += __shfl_xor_sync(0xffffffffu, cnt_cry, o);
-                cnt_hole += __shfl_xor_sync(0xffffffffu, cnt_hole, o);
-                cnt_cone += __shfl_xor_sync(0xffffffffu, cnt_cone, o);
+                counts.rays += __shfl_xor_sync(0xffffffffu, counts.rays, o);
+                counts.crystal += __shfl_xor_sync(0xffffffffu, counts.crystal, o);
+                counts.hole += __shfl_xor_sync(0xffffffffu, counts.hole, o);
+                counts.cone += __shfl_xor_sync(0xffffffffu, counts.cone, o);
             }
             if (lane == 0) {
-                atomicAdd(&P.counters[0], cnt_rays);
-                atomicAdd(&P.counters[1], cnt_cry);
-                atomicAdd(&P.counters[2], cnt_hole);
-                atomicAdd(&P.counters[3], cnt_cone);
+                atomicAdd(&P.counters[0], counts.rays);
+                atomicAdd(&P.counters[1], counts.crystal);
+                atomicAdd(&P.counters[2], counts.hole);
+                atomicAdd(&P.counters[3], counts.cone);
             }
         }
     }
@@ -1219,13 +1221,13 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
     }
 }
 
-template <bool RECORD, bool FEW>
+template <bool RECORD, bool FEW, bool COUNT>
 __global__ void __launch_bounds__(kPeThreads, 2) pe_trace_kernel(const __grid_constant__ PEParams P,
                                                                 const __grid_constant__ DevGeometry G) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PeSmem& S = *reinterpret_cast<PeSmem*>(smem_raw);
     const long long tile = P.tile_list ? P.tile_list[blockIdx.x] : (long long)blockIdx.x;
-    pe_tile<RECORD, FEW>(P, G, S, tile);
+    pe_tile<RECORD, FEW, COUNT>(P, G, S, tile);
 }
 
 // The batch's geometries, in constant memory: the tile code reads launch
@@ -1260,8 +1262,8 @@ __global__ void __launch_bounds__(kPeThreads, 2) pe_batch_kernel(int n_geoms, lo
         const long long item = s_item;
         const int g = s_geom;
         if (item >= total) break;
-        if (c_batch[g].P.pair > 1) pe_tile<false, true>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
-        else pe_tile<false, false>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
+        if (c_batch[g].P.pair > 1) pe_tile<false, true, false>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
+        else pe_tile<false, false, false>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
         __syncthreads();
     }
 }
@@ -1273,7 +1275,7 @@ size_t pe_smem_bytes() { return sizeof(PeSmem); }
 // The dynamic shared memory limit is a per-device function attribute: set it
 // once per (device, kernel).
 static cudaError_t allow_smem(const void* fn, int which) {
-    static unsigned long long done[4] = {0, 0, 0, 0};
+    static unsigned long long done[6] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1292,8 +1294,11 @@ cudaError_t pe_launch(const PEParams& p, const DevGeometry& geo, bool record, lo
         if (e == cudaSuccess) kernel<<<(unsigned)n_tiles, kPeThreads, smem, stream>>>(p, geo);
         return e;
     };
-    const cudaError_t e = record ? launch(pe_trace_kernel<true, false>, 0)
-                                 : (p.pair > 1 ? launch(pe_trace_kernel<false, true>, 3) : launch(pe_trace_kernel<false, false>, 1));
+    // counting instantiations of their own: the counters take 14 registers of the loop
+    cudaError_t e;
+    if (record) e = launch(pe_trace_kernel<true, false, false>, 0);
+    else if (p.counters) e = p.pair > 1 ? launch(pe_trace_kernel<false, true, true>, 5) : launch(pe_trace_kernel<false, false, true>, 4);
+    else e = p.pair > 1 ? launch(pe_trace_kernel<false, true, false>, 3) : launch(pe_trace_kernel<false, false, false>, 1);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
