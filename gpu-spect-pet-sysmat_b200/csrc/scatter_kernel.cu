@@ -456,7 +456,7 @@ __global__ void scatter_transfer_kernel(ScatterParams P, DevGeometry G, ScatterT
 #pragma unroll
                     for (int j = 0; j < kMaxAnchorsPerPass; ++j)
                         if (use[j])
-                            acc[j] += scatter_term<false>(P, D, C, kn, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
+                            acc[j] += scatter_term<false>(P, D, C, kn, nullptr, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
                                                    Is[j].z);
                 }
             }
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(kTrRanks * kTrSrcs) scatter_transfer_tiled_ker
 #pragma unroll
                 for (int j = 0; j < kMaxAnchorsPerPass; ++j)
                     if (use[j])
-                        acc[j] += scatter_term<false>(P, D, C, kn, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
+                        acc[j] += scatter_term<false>(P, D, C, kn, nullptr, T.kn_inv_norm, I[j].x, I[j].y, I[j].z, Is[j].x, Is[j].y,
                                                Is[j].z);
             }
         }
@@ -829,7 +829,7 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
                 const float isx = (V.x - D.x) * D.cm - (V.z - D.z) * D.sm;
                 const float isy = V.y - D.y;
                 const float isz = (V.x - D.x) * D.sm + (V.z - D.z) * D.cm;
-                const float t = scatter_term<true>(P, D, c, S.kn, T.kn_inv_norm, V.x, V.y, V.z, isx, isy, isz);
+                const float t = scatter_term<true>(P, D, c, S.kn, T.erfc, T.kn_inv_norm, V.x, V.y, V.z, isx, isy, isz);
                 add = (double)(S.wgt[slot][col][j] * t);
             }
             // a cell may wait for several points: one point at a time
