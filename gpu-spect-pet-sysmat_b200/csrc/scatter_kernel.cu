@@ -586,7 +586,7 @@ struct __align__(16) ScSmem {
     float scale[kScTileD];                             // per detector: mu_c / mu_pe / points, or plate mu_c / mu_t
     int d[kScTileD];
     unsigned todo[ScShape<C>::NQ][C];                  // per (point, column): detectors that pass the column's cull
-    unsigned short queue[kScWarps][64];                // point << 10 | detector << 5 | voxel
+    unsigned short queue[kScWarps][96];                // point << 10 | detector << 5 | voxel
 };
 
 template <int C>
@@ -666,6 +666,8 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
         const BrickCol bc = brick_column(P, b, c0 + w_col);
         if (bc.valid && y0 + w_y < P.ny) w_at = bc.x + (long long)P.nx * (y0 + w_y + (long long)P.ny * bc.z);
     }
+    const unsigned below = (1u << lane) - 1u;
+    unsigned short* const waiting = S.queue[warp];
     long long pair_at = 0;                                   // this lane's pair column
     if (lane < n_det) {
         const int rank = P.rank0 + dt * kScTileD + lane;
@@ -763,12 +765,12 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
         int count = 0;                                       // queue length
         int k = 0;                                           // point of the batch
         unsigned todo = 0u;                                  // its detectors still to test
-        float ax = 0.0f, ay = 0.0f, az = 0.0f, inv_a = 0.0f;
-        bool live = false;
+        float ux = 0.0f, uy = 0.0f, uz = 0.0f;               // direction voxel -> point, NaN where the voxel has no term
         auto open_point = [&] {
             // weights and directions of the voxels (lane)
             const float4 pt = S.src[k];
             float w;
+            bool live;
             if (KIND == kScatterCrystal) {
                 w = S.wgt[k][col][lane];
                 live = w != 0.0f;
@@ -784,8 +786,9 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
                 live = I.w >= 0.0f;
             }
             todo = __any_sync(0xffffffffu, live) ? S.todo[k][col] & mine : 0u;
-            ax = pt.x - I.x; ay = pt.y - I.y; az = pt.z - I.z;
-            inv_a = fast_rsqrt(fmaf(ax, ax, fmaf(ay, ay, az * az)));
+            ux = pt.x - I.x; uy = pt.y - I.y; uz = pt.z - I.z;
+            const float inv = live ? fast_rsqrt(fmaf(ux, ux, fmaf(uy, uy, uz * uz))) : __int_as_float(0x7fffffff);
+            ux *= inv; uy *= inv; uz *= inv;
         };
         open_point();
         for (;;) {
@@ -796,18 +799,25 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
                     open_point();
                     continue;
                 }
-                const int dl = __ffs(todo) - 1;
+                // two detectors at a time (the second may be the first again: then it passes nothing)
+                const int d0 = __ffs(todo) - 1;
                 todo &= todo - 1u;
-                const float4 bd = S.b[k][dl];
-                const bool pass = live && fmaf(ax, bd.x, fmaf(ay, bd.y, az * bd.z)) * inv_a > bd.w;
-                const unsigned m = __ballot_sync(0xffffffffu, pass);
-                if (pass) S.queue[warp][count + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(k << 10 | dl << 5 | lane);
-                count += __popc(m);
+                const bool both = todo != 0u;
+                const int d1 = both ? __ffs(todo) - 1 : d0;
+                todo &= todo - 1u;
+                const float4 b0 = S.b[k][d0], b1 = S.b[k][d1];
+                const bool p0 = fmaf(ux, b0.x, fmaf(uy, b0.y, uz * b0.z)) > b0.w;
+                const bool p1 = both && fmaf(ux, b1.x, fmaf(uy, b1.y, uz * b1.z)) > b1.w;
+                const unsigned m0 = __ballot_sync(0xffffffffu, p0), m1 = __ballot_sync(0xffffffffu, p1);
+                if (p0) waiting[count + __popc(m0 & below)] = (unsigned short)(k << 10 | d0 << 5 | lane);
+                count += __popc(m0);
+                if (p1) waiting[count + __popc(m1 & below)] = (unsigned short)(k << 10 | d1 << 5 | lane);
+                count += __popc(m1);
             }
             if (count == 0) break;
             __syncwarp();
             const int n = min(count, 32);
-            const unsigned item = S.queue[warp][lane < n ? lane : 0];
+            const unsigned item = waiting[lane < n ? lane : 0];
             const int slot = item >> 10, dl = item >> 5 & 31, j = item & 31;
             double add = 0.0;
             if (lane < n) {
@@ -839,9 +849,10 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
                 __syncwarp();
             }
             // the rest of the queue moves up
-            const unsigned short rest = S.queue[warp][32 + lane];
+            const unsigned short rest = waiting[32 + lane], more = waiting[64 + lane];
             __syncwarp();
-            if (lane < count - n) S.queue[warp][lane] = rest;
+            if (lane < count - n) waiting[lane] = rest;
+            if (lane + 32 < count - n) waiting[32 + lane] = more;
             count -= n;
         }
     }
