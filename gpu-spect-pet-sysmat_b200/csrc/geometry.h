@@ -70,10 +70,12 @@ struct HostGeometry {
     std::vector<int> h_plate;
     PlateBox plate[kMaxPlates];
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};   // box of the crystals
+    bool rotated = true;                          // some crystal's frame is not the world's
 };
 
-// Grows the crystals' box by crystal d's.
-inline void add_crystal_box(HostGeometry* g, int d, const float lo[3], const float hi[3]) {
+// Takes crystal d, of box lo .. hi and rotation cos, sin, into the fields about all of them.
+inline void add_crystal(HostGeometry* g, int d, const float lo[3], const float hi[3], float cosine, float sine) {
+    g->rotated = (d > 0 && g->rotated) || cosine != 1.0f || sine != 0.0f;
     for (int a = 0; a < 3; ++a) {
         if (d == 0 || lo[a] < g->lo[a]) g->lo[a] = lo[a];
         if (d == 0 || hi[a] > g->hi[a]) g->hi[a] = hi[a];

@@ -60,6 +60,7 @@ void pe_plan(const HostGeometry& g, const int sv[3], const int sc[3], const int 
         }
     }
     if (P.pair > 1) P.group = P.pair * P.n_sv;
+    P.rotated = g.rotated;
     P.inv_sv = 1.0f / (float)P.n_sv;
     // Range S of the coordinates a ray spans: the image (any rotation) and the crystals.
     const float half[3] = {g.nx * g.voxel[0] * 0.5f + std::fabs(g.shift[0]), g.ny * g.voxel[1] * 0.5f + std::fabs(g.shift[1]),

@@ -440,7 +440,7 @@ struct RayCounts {
 // either way, so the cone test (`csp`: the sub-point's ConeSelf) is taken only
 // for candidates with a nonzero chord.  Returns the contribution; in RECORD
 // mode also the hit record.
-template <bool RECORD, bool FEW, bool COUNT>
+template <bool RECORD, bool FEW, bool ROT, bool COUNT>
 __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry& G, const PeSmem& S,
                                            const WarpLists& L, unsigned plates_sure, bool any_hole,
                                            const float4* csp, const Detecting& D, const Vec3& p,
@@ -508,63 +508,99 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
         if ((through - in_holes) >= 0.00001f) att += pb.mu_total * (through - in_holes);
     }
     // Other crystals among the candidates, each in its own frame (:687-725).
+    // `f` and `len`: chord_quick's call in the world's frame, -1 for a rotated crystal.
+    auto settle = [&](int e, const float4& kp, const float4& kh, int f, float len) {
+        const int k = e & kIndex;
+        float kc = 1.0f, ks = 0.0f;               // cos, sin of the crystal's rotation
+        float kix = 0.0f, kiz = 0.0f;             // 1 / extents in its frame
+        if (!ROT || !(e & kRotated)) {
+            if (f < 0 && cr.ok) f = chord_filter(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, P.chord_delta, &len);
+        } else {
+            kc = S.c_lo[k].w;
+            ks = S.c_hi[k].w;
+            // the segment in the crystal's frame; its rotation rounds once more, hence twice the margin
+            const float px = p.x - kp.x, pz = p.z - kp.z;
+            const ChordRay kr = make_chord_ray(fmaf(px, kc, -pz * ks), p.y - kp.y, fmaf(px, ks, pz * kc),
+                                               fmaf(dxw, kc, -dzw * ks), dy, fmaf(dxw, ks, dzw * kc), r,
+                                               2.0f * P.chord_delta);
+            kix = kr.ix;
+            kiz = kr.iz;
+            f = chord_quick(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, &len);
+            if (f < 0 && kr.ok)
+                f = chord_filter(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, 2.0f * P.chord_delta, &len);
+        }
+        if (COUNT && f) ++n.crystal;
+        if (!f) return;
+        if (f < 0) {
+            len = crystal_chord_exact(p, q, kp, kh, kc, ks);
+            if (len == 0.0f) return;
+        } else if (FEW) {
+            // Entries of few rays keep the exact form's rounding (their matrices feed the
+            // scatter pipeline, whose bf16 operands and error estimates magnify it); entries
+            // of many rays average the filter's, which is of the same size.
+            const float ax = p.x - kp.x, az = p.z - kp.z, bx = q.x - kp.x, bz = q.z - kp.z;
+            if (!ROT || !(e & kRotated))
+                len = chord_value(ax, p.y - kp.y, az, bx, q.y - kp.y, bz, kh.x, kh.y, kh.z, cr.ix, cr.iy, cr.iz, inv_r);
+            else
+                len = chord_value(ax * kc - az * ks, p.y - kp.y, ax * ks + az * kc, bx * kc - bz * ks, q.y - kp.y,
+                                  bx * ks + bz * kc, kh.x, kh.y, kh.z, kix, cr.iy, kiz, inv_r);
+        }
+        if (!(e & kConeSure)) {
+            if (COUNT) ++n.cone;
+            const ConeSelf cs = cone_of<FEW>(csp, D, p);
+            int g = cone_filter(cs, p, kp.x, kp.y, kp.z, kh.w);
+            if (g < 0) g = cone_crystal_exact(cs, p, kp.x, kp.y, kp.z, 2.0f * kh.w) ? 1 : 0;
+            if (!g) return;
+        }
+        att += len * kp.w;
+        if (RECORD && len > 0.0f) {
+            if (rec_c < kRecCrystals) rec[3 + kRecHoles + rec_c] = S.c_id[k];
+            else atomicOr(status, kStatusRecordOverflow);
+            ++rec_c;
+        }
+    };
     const int nwc = (L.n_c + 31) >> 5;
     for (int wd = 0; wd < nwc; ++wd) {
         unsigned bits = L.pass_c[wd];
         while (bits) {
-            const int b = __ffs(bits) - 1;
+            if (FEW || ROT || RECORD) {
+                const int b = __ffs(bits) - 1;
+                bits &= bits - 1;
+                const int e = L.list_c[(wd << 5) + b], k = e & kIndex;
+                const float4 kp = S.c_pos[k], kh = S.c_half[k];
+                float len = 0.0f;
+                int f = -1;
+                if (!ROT || !(e & kRotated)) f = chord_quick(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, &len);
+                if (ROT || f) settle(e, kp, kh, f, len);
+                continue;
+            }
+            // Two candidates at a time: their tests are independent chains of dependent
+            // instructions, whose latency the 16 warps of an SM do not hide (two plates of
+            // 20x20 holes, 6400 crystals: 177 -> 155 ms).  Entries of few rays, whose hits go
+            // through the longer chord_value, and rotated frames ran 2 to 20 % slower in pairs.
+            const int b0 = __ffs(bits) - 1;
             bits &= bits - 1;
-            const int e = L.list_c[(wd << 5) + b], k = e & kIndex;
-            const float4 kp = S.c_pos[k], kh = S.c_half[k];
-            float len = 0.0f, kc = 1.0f, ks = 0.0f;   // cos, sin of the crystal's rotation
-            float kix = 0.0f, kiz = 0.0f;             // 1 / extents in its frame
-            int f;
-            if (!(e & kRotated)) {
-                f = chord_quick(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, &len);
-                if (f < 0) f = chord_filter(cr, kp.x, kp.y, kp.z, kh.x, kh.y, kh.z, P.chord_delta, &len);
-            } else {
-                kc = S.c_lo[k].w;
-                ks = S.c_hi[k].w;
-                // the segment in the crystal's frame; its rotation rounds once more, hence twice the margin
-                const float px = p.x - kp.x, pz = p.z - kp.z;
-                const ChordRay kr = make_chord_ray(fmaf(px, kc, -pz * ks), p.y - kp.y, fmaf(px, ks, pz * kc),
-                                                   fmaf(dxw, kc, -dzw * ks), dy, fmaf(dxw, ks, dzw * kc), r,
-                                                   2.0f * P.chord_delta);
-                kix = kr.ix;
-                kiz = kr.iz;
-                f = kr.ok ? chord_quick(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, &len) : -1;
-                if (f < 0 && kr.ok)
-                    f = chord_filter(kr, 0.0f, 0.0f, 0.0f, kh.x, kh.y, kh.z, 2.0f * P.chord_delta, &len);
+            const int b1 = bits ? __ffs(bits) - 1 : b0;
+            const bool two = bits != 0u;
+            bits &= bits - 1;
+            const int e0 = L.list_c[(wd << 5) + b0], e1 = L.list_c[(wd << 5) + b1];
+            const float4 kp0 = S.c_pos[e0 & kIndex], kh0 = S.c_half[e0 & kIndex];
+            const float4 kp1 = S.c_pos[e1 & kIndex], kh1 = S.c_half[e1 & kIndex];
+            float len0, len1;
+            int f0 = chord_quick(cr, kp0.x, kp0.y, kp0.z, kh0.x, kh0.y, kh0.z, &len0);
+            int f1 = chord_quick(cr, kp1.x, kp1.y, kp1.z, kh1.x, kh1.y, kh1.z, &len1);
+            if (!two) f1 = 0;
+            if (!(f0 | f1)) continue;
+            if ((f0 | f1) > 0 && !(f0 && !(e0 & kConeSure)) && !(f1 && !(e1 & kConeSure))) {
+                if (f0) att += len0 * kp0.w;
+                if (f1) att += len1 * kp1.w;
+                if (COUNT) n.crystal += f0 + f1;
+                continue;
             }
-            if (COUNT && f) ++n.crystal;
-            if (f < 0 || !cr.ok) {
-                len = crystal_chord_exact(p, q, kp, kh, kc, ks);
-                f = len != 0.0f;
-            }
-            if (!f) continue;
-            if (FEW && f > 0 && cr.ok) {
-                // Entries of few rays keep the exact form's rounding (their matrices feed the
-                // scatter pipeline, whose bf16 operands and error estimates magnify it); entries
-                // of many rays average the filter's, which is of the same size.
-                const float ax = p.x - kp.x, az = p.z - kp.z, bx = q.x - kp.x, bz = q.z - kp.z;
-                if (!(e & kRotated))
-                    len = chord_value(ax, p.y - kp.y, az, bx, q.y - kp.y, bz, kh.x, kh.y, kh.z, cr.ix, cr.iy, cr.iz, inv_r);
-                else
-                    len = chord_value(ax * kc - az * ks, p.y - kp.y, ax * ks + az * kc, bx * kc - bz * ks, q.y - kp.y,
-                                      bx * ks + bz * kc, kh.x, kh.y, kh.z, kix, cr.iy, kiz, inv_r);
-            }
-            if (!(e & kConeSure)) {
-                if (COUNT) ++n.cone;
-                const ConeSelf cs = cone_of<FEW>(csp, D, p);
-                int g = cone_filter(cs, p, kp.x, kp.y, kp.z, kh.w);
-                if (g < 0) g = cone_crystal_exact(cs, p, kp.x, kp.y, kp.z, 2.0f * kh.w) ? 1 : 0;
-                if (!g) continue;
-            }
-            att += len * kp.w;
-            if (RECORD && len > 0.0f) {
-                if (rec_c < kRecCrystals) rec[3 + kRecHoles + rec_c] = S.c_id[k];
-                else atomicOr(status, kStatusRecordOverflow);
-                ++rec_c;
+#pragma unroll 1
+            for (int u = 0; u < 2; ++u) {
+                const int e = u ? e1 : e0, f = u ? f1 : f0;
+                if (f) settle(e, S.c_pos[e & kIndex], S.c_half[e & kIndex], f, u ? len1 : len0);
             }
         }
     }
@@ -575,7 +611,7 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
         if (plate_miss) return 0.0f;
     }
 
-    return ray_value(D, FEW || D.rotated, ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
+    return ray_value(D, FEW || (ROT && D.rotated), ps, xDs, yDs, zDs, att, r, inv_r, cr, dxw, dy, dzw);
 }
 
 // One ray with its candidates read straight from the geometry tables: every
@@ -709,7 +745,7 @@ __device__ __forceinline__ int warp_append(bool pass, int value, unsigned short*
 
 // One tile (8 crystals x one voxel brick) of geometry G.  Shared by the
 // one-launch-per-geometry kernel and the persistent batch kernel.
-template <bool RECORD, bool FEW, bool COUNT>
+template <bool RECORD, bool FEW, bool ROT, bool COUNT>
 __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G, PeSmem& S, long long tile) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
@@ -982,7 +1018,7 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                             const float4 kp = S.c_pos[k];
                             const bool sure = pass && flag_sure && cone_sure(mid, rho, kp.x, kp.y, kp.z, S.c_half[k].w,
                                                                              D.cx, D.cy, D.cz, 0.5f * D.crit);
-                            if (S.c_lo[k].w != 1.0f || S.c_hi[k].w != 0.0f) k |= kRotated;
+                            if (ROT && (S.c_lo[k].w != 1.0f || S.c_hi[k].w != 0.0f)) k |= kRotated;
                             if (sure) k |= kConeSure;
                         }
                         cnt = warp_append(pass, k, L.list_c, cnt, kListC, lane);
@@ -1153,14 +1189,14 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                                 if (!FEW) p = subpoint_of(P, ix, iy, iz, s0 + j);
                                 // ... in the detecting crystal's frame
                                 Vec3 ps{p.x - D.cx, p.y - D.cy, p.z - D.cz};
-                                if (D.rotated) ps = Vec3{ps.x * D.cm - ps.z * D.sm, ps.y, ps.x * D.sm + ps.z * D.cm};
+                                if (ROT && D.rotated) ps = Vec3{ps.x * D.cm - ps.z * D.sm, ps.y, ps.x * D.sm + ps.z * D.cm};
                                 int* rec = nullptr;
                                 if (RECORD) {
                                     const int c = (sz * P.dX + sx) * P.dY + sy;   // the oracle's sub-cell order
                                     rec = P.rec_out + ((long long)rec_slot * P.n_sv * P.n_sc + (long long)(s0 + j) * P.n_sc + c) *
                                                           kRecWords;
                                 }
-                                const float v = trace_ray<RECORD, FEW, COUNT>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
+                                const float v = trace_ray<RECORD, FEW, ROT, COUNT>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
                                                                   P.status, counts);
                                 if (COUNT) ++counts.rays;
                                 // Kahan summation of the lane's rays.
@@ -1221,13 +1257,13 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
     }
 }
 
-template <bool RECORD, bool FEW, bool COUNT>
+template <bool RECORD, bool FEW, bool ROT, bool COUNT>
 __global__ void __launch_bounds__(kPeThreads, 2) pe_trace_kernel(const __grid_constant__ PEParams P,
                                                                 const __grid_constant__ DevGeometry G) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PeSmem& S = *reinterpret_cast<PeSmem*>(smem_raw);
     const long long tile = P.tile_list ? P.tile_list[blockIdx.x] : (long long)blockIdx.x;
-    pe_tile<RECORD, FEW, COUNT>(P, G, S, tile);
+    pe_tile<RECORD, FEW, ROT, COUNT>(P, G, S, tile);
 }
 
 // The batch's geometries, in constant memory: the tile code reads launch
@@ -1262,8 +1298,15 @@ __global__ void __launch_bounds__(kPeThreads, 2) pe_batch_kernel(int n_geoms, lo
         const long long item = s_item;
         const int g = s_geom;
         if (item >= total) break;
-        if (c_batch[g].P.pair > 1) pe_tile<false, true, false>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
-        else pe_tile<false, false, false>(c_batch[g].P, c_batch[g].G, S, item - c_batch[g].tile_begin);
+        const PeBatchGeom& it = c_batch[g];
+        const long long tile = item - it.tile_begin;
+        if (it.P.pair > 1) {
+            if (it.P.rotated) pe_tile<false, true, true, false>(it.P, it.G, S, tile);
+            else pe_tile<false, true, false, false>(it.P, it.G, S, tile);
+        } else {
+            if (it.P.rotated) pe_tile<false, false, true, false>(it.P, it.G, S, tile);
+            else pe_tile<false, false, false, false>(it.P, it.G, S, tile);
+        }
         __syncthreads();
     }
 }
@@ -1275,7 +1318,7 @@ size_t pe_smem_bytes() { return sizeof(PeSmem); }
 // The dynamic shared memory limit is a per-device function attribute: set it
 // once per (device, kernel).
 static cudaError_t allow_smem(const void* fn, int which) {
-    static unsigned long long done[6] = {};
+    static unsigned long long done[8] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1294,11 +1337,17 @@ cudaError_t pe_launch(const PEParams& p, const DevGeometry& geo, bool record, lo
         if (e == cudaSuccess) kernel<<<(unsigned)n_tiles, kPeThreads, smem, stream>>>(p, geo);
         return e;
     };
-    // counting instantiations of their own: the counters take 14 registers of the loop
+    // Counting instantiations of their own: the counters take 14 registers of the loop.
+    // Detectors without a rotated crystal, the usual ones, leave the frames' code out: a
+    // sweep of 40 entries of 16 rays 319 -> 288 ms, 64-ray entries 8.3 -> 7.5 ms.
     cudaError_t e;
-    if (record) e = launch(pe_trace_kernel<true, false, false>, 0);
-    else if (p.counters) e = p.pair > 1 ? launch(pe_trace_kernel<false, true, true>, 5) : launch(pe_trace_kernel<false, false, true>, 4);
-    else e = p.pair > 1 ? launch(pe_trace_kernel<false, true, false>, 3) : launch(pe_trace_kernel<false, false, false>, 1);
+    if (record) e = launch(pe_trace_kernel<true, false, true, false>, 0);
+    else if (p.counters)
+        e = p.pair > 1 ? launch(pe_trace_kernel<false, true, true, true>, 1) : launch(pe_trace_kernel<false, false, true, true>, 2);
+    else if (p.rotated)
+        e = p.pair > 1 ? launch(pe_trace_kernel<false, true, true, false>, 3) : launch(pe_trace_kernel<false, false, true, false>, 4);
+    else
+        e = p.pair > 1 ? launch(pe_trace_kernel<false, true, false, false>, 5) : launch(pe_trace_kernel<false, false, false, false>, 6);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
@@ -1307,7 +1356,7 @@ cudaError_t pe_batch_launch(const PeBatchGeom* geoms, int n_geoms, long long tot
                             int grid, cudaStream_t stream) {
     if (total <= 0) return cudaSuccess;
     if (n_geoms < 1 || n_geoms > kBatchConst) return cudaErrorInvalidValue;
-    cudaError_t e = allow_smem((const void*)pe_batch_kernel, 2);
+    cudaError_t e = allow_smem((const void*)pe_batch_kernel, 7);
     if (e != cudaSuccess) return e;
     e = cudaMemcpyToSymbolAsync(c_batch, geoms, sizeof(PeBatchGeom) * (size_t)n_geoms, 0, cudaMemcpyDeviceToDevice,
                                 stream);
@@ -1320,7 +1369,7 @@ cudaError_t pe_batch_launch(const PeBatchGeom* geoms, int n_geoms, long long tot
 
 int pe_batch_blocks_per_sm() {
     int n = 0;
-    if (allow_smem((const void*)pe_batch_kernel, 2) != cudaSuccess) return 1;
+    if (allow_smem((const void*)pe_batch_kernel, 7) != cudaSuccess) return 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pe_batch_kernel, kPeThreads, sizeof(PeSmem)) != cudaSuccess)
         return 1;
     return n > 0 ? n : 1;

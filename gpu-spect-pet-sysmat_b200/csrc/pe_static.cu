@@ -181,7 +181,7 @@ int derive_into_stage(const float* col, size_t n_col, const float* det, size_t n
         float* hi = c_hi + 4 * (size_t)d;
         lo[0] = D[1] - ex; lo[1] = cy - t / 2.0f; lo[2] = D[3] - ez; lo[3] = 0.0f;
         hi[0] = D[1] + ex; hi[1] = cy + t / 2.0f; hi[2] = D[3] + ez; hi[3] = 0.0f;
-        add_crystal_box(&g, d, lo, hi);
+        add_crystal(&g, d, lo, hi, cm, sm);
     }
     return SM_OK;
 }

@@ -246,7 +246,7 @@ struct ChordRay {
     float px, py, pz;
     float ix, iy, iz, ax, ay, az;
     float len;
-    float margin;   // largest of delta |1/d_i|
+    float margin;   // largest of delta |1/d_i|; infinite unless ok: then nothing is clear to chord_quick
     float eps;      // the reference's 0.001 in units of the segment
     bool ok;        // no axis is near the reference's degenerate extent (0.001)
 };
@@ -264,9 +264,9 @@ SM_HD ChordRay make_chord_ray(float px, float py, float pz, float dx, float dy, 
     c.ix = chord_rcp(dx); c.iy = chord_rcp(dy); c.iz = chord_rcp(dz);
     c.ax = fabsf(c.ix); c.ay = fabsf(c.iy); c.az = fabsf(c.iz);
     c.len = len;
-    c.margin = delta * fmaxf(fmaxf(c.ax, c.ay), c.az);
-    c.eps = 0.001f * chord_rcp(len);
     c.ok = fminf(fminf(fabsf(dx), fabsf(dy)), fabsf(dz)) > 0.002f;
+    c.margin = c.ok ? delta * fmaxf(fmaxf(c.ax, c.ay), c.az) : INFINITY;
+    c.eps = 0.001f * chord_rcp(len);
     return c;
 }
 
