@@ -27,7 +27,7 @@ namespace smb {
 
 constexpr int kKnNodes = 512;            // Klein-Nishina table: nodes j * pi / 512, j = 0..512
 constexpr int kScTileD = 32;             // detectors per CTA (one per lane)
-constexpr int kScBrickX = 8;             // voxel brick: 8 (x) x 32 (y) x 1 (z); a CTA takes 8, 4, 2 or 1 of its columns
+constexpr int kScBrickX = 8;             // voxel brick: 8 (x) x 32 (y) x 1 (z); a CTA takes 4, 2 or 1 of its columns
 constexpr int kScBrickY = 32;
 constexpr int kScWarps = 8;
 constexpr int kScThreads = 32 * kScWarps;

@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(kTrRanks * kTrSrcs) scatter_transfer_tiled_ker
 }
 
 // ---- exact scatter of a detector tile and a voxel brick -----------------------------------
-// CTA = 32 detectors x C columns (C = 8, 4, 2 or 1) of 32 voxels along y, 8 warps; 8 / C
+// CTA = 32 detectors x C columns (C = 4, 2 or 1) of 32 voxels along y, 8 warps; 8 / C
 // warps share a column and take every (8 / C)-th detector.  Only a few per cent of the
 // (detector, voxel, scatter point) terms pass the energy window, scattered over lanes, and
 // a term costs some 500 instructions: each warp lists the pairs that can pass and evaluates
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kTrRanks * kTrSrcs) scatter_transfer_tiled_ker
 // registers and shared memory alike.
 template <int C>
 struct ScShape {
-    static constexpr int NQ = C == 8 ? 4 : 8;          // points per batch (shared memory: 5 KB each)
+    static constexpr int NQ = 8;                       // points per batch (shared memory: 5 KB each)
     static constexpr int W = kScWarps / C;             // warps per column
     static constexpr int PER = NQ * 32 * C / kScThreads;   // staged weights per thread
 };
@@ -591,7 +591,7 @@ struct __align__(16) ScSmem {
 
 template <int C>
 constexpr bool two_ctas() { return 2 * (sizeof(ScSmem<C>) + 1024) <= 228 * 1024; }
-static_assert(two_ctas<8>() && two_ctas<4>() && two_ctas<2>() && two_ctas<1>(), "two CTAs per SM");
+static_assert(two_ctas<4>() && two_ctas<2>() && two_ctas<1>(), "two CTAs per SM");
 
 // scatter_term's view of a staged (point, detector).
 struct SrcView {
@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
     const float col_ex = -P.sin_a, col_ey = P.cos_a;
     const float col_t = (float)(min(kScBrickY, P.ny - y0) - 1) * P.vy;
     const float c_cut = S.det[3][lane].z;                    // lane = detector
-    const unsigned mine = W == 1 ? 0xffffffffu : (W == 2 ? 0x55555555u : (W == 4 ? 0x11111111u : 0x01010101u)) << sub;
+    const unsigned mine = (W == 2 ? 0x55555555u : (W == 4 ? 0x11111111u : 0x01010101u)) << sub;
 
     // This thread's place in the staged weights: one voxel of the tile, points first, first + step, ...
     constexpr int kPlaces = 32 * C, kStep = kScThreads / kPlaces;
@@ -972,17 +972,28 @@ cudaError_t launch_scatter_main(const ScatterParams& P, const DevGeometry& G, co
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    // Fewer columns per CTA repeat the staging and the culls; they pay while the CTAs
-    // would fill less than four waves of the device (2 per SM).
-    const long long want = 8LL * sms;
-    const int c = tiles >= want ? 8 : (2 * tiles >= want ? 4 : (4 * tiles >= want ? 2 : 1));
+    // Columns per CTA: fewer repeat the staging and the culls (by 1.12 and 1.37 of a
+    // column's time at 2048 crystals), more leave the last wave of CTAs (2 per SM) emptier.
+    // The cheaper of those that fill two waves, else one column.  (Eight columns: no faster
+    // anywhere, 142.7 against 142.2 ms for 2048 crystals, 29.0 against 25.4 ms for 576.)
+    const long long slots = 2LL * sms;
+    int c = 1;
+    double best = 0.0;
+    for (int n : {4, 2, 1}) {
+        const long long blocks = tiles * (kScBrickX / n);
+        if (blocks < 2 * slots) continue;
+        const double waves = (double)((blocks + slots - 1) / slots);
+        const double cost = waves * n * (n == 4 ? 1.0 : (n == 2 ? 1.12 : 1.37));
+        if (best == 0.0 || cost < best) {
+            best = cost;
+            c = n;
+        }
+    }
     if (P.kind == kScatterCrystal) {
-        if (c == 8) return launch_main<kScatterCrystal, 8>(P, G, T, tiles, s);
         if (c == 4) return launch_main<kScatterCrystal, 4>(P, G, T, tiles, s);
         if (c == 2) return launch_main<kScatterCrystal, 2>(P, G, T, tiles, s);
         return launch_main<kScatterCrystal, 1>(P, G, T, tiles, s);
     }
-    if (c == 8) return launch_main<kScatterCollimator, 8>(P, G, T, tiles, s);
     if (c == 4) return launch_main<kScatterCollimator, 4>(P, G, T, tiles, s);
     if (c == 2) return launch_main<kScatterCollimator, 2>(P, G, T, tiles, s);
     return launch_main<kScatterCollimator, 1>(P, G, T, tiles, s);

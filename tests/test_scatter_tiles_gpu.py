@@ -1,4 +1,4 @@
-"""The exact scatter kernel's split into CTAs of 8, 4, 2 or 1 voxel columns: every split
+"""The exact scatter kernel's split into CTAs of 4, 2 or 1 voxel columns: every split
 gives the same bits.  The sizes cross each line of the dispatch (rows x bricks), with a
 ragged last detector tile, brick and y run; the values themselves are checked against the
 reference's and the oracle's in test_scatter_gpu.py."""
@@ -25,7 +25,7 @@ def full():
 
 
 @pytest.mark.parametrize("part", ["crystal", "collimator"])
-@pytest.mark.parametrize("rows", [(700, 1403), (33, 350), (1024, 1200), (2047, 2048)])   # 4, 2, 1 and 1 columns
+@pytest.mark.parametrize("rows", [(700, 1403), (33, 350), (1024, 1200), (2047, 2048)])   # 4, 4, 2 and 1 columns
 def test_every_split_gives_the_same_bits(full, part, rows):
     geo, pe, matrix = full
     assert np.isfinite(matrix[part]).all() and (matrix[part] > 0).any()
