@@ -53,7 +53,7 @@ struct PEParams {
     float* dst;
     long long ld;
     int* status;
-    unsigned long long* counters; // optional: rays, exact crystal tests, exact hole tests, cone tests
+    unsigned long long* counters; // optional: rays, crystals and holes crossed or tested exactly, cone tests
     // record mode
     int rec_n;
     const long long* rec_rows;
@@ -95,7 +95,8 @@ constexpr int kBatchConst = 64;   // geometries per persistent launch (constant-
 // One persistent launch over `total` items of n_geoms <= kBatchConst
 // geometries (device table `geoms`, ordered by tile_begin, first item 0):
 // copies the table to constant memory, zeroes `counter`, launches.
-cudaError_t pe_batch_launch(const PeBatchGeom* geoms, int n_geoms, long long total, unsigned long long* counter,
+int pe_batch_form(const PEParams& p);   // 0 .. 3: which kernel traces it; the geometries of a launch share it
+cudaError_t pe_batch_launch(const PeBatchGeom* geoms, int n_geoms, int form, long long total, unsigned long long* counter,
                             int grid, cudaStream_t stream);
 int pe_batch_blocks_per_sm();
 

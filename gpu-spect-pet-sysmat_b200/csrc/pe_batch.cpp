@@ -37,7 +37,7 @@ struct sm_pe_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     struct Chunk {
-        int first, count;
+        int first, count, form;
         long long items;
     };
     std::vector<Chunk> chunks;
@@ -249,9 +249,10 @@ int sm_pe_batch_create(sm_context* ctx, int n, const sm_geometry* const* geos, c
         b.G = geo->dev.view;
         order.push_back({est_cost(g, b.P) / std::max<long long>(1, b.P.n_tiles), i});
     }
-    // most expensive tiles first
-    std::stable_sort(order.begin(), order.end(), [](const std::pair<double, int>& a, const std::pair<double, int>& b) {
-        return a.first > b.first;
+    // by form, then most expensive tiles first
+    std::stable_sort(order.begin(), order.end(), [&](const std::pair<double, int>& a, const std::pair<double, int>& b) {
+        const int fa = pe_batch_form(items[a.second].P), fb = pe_batch_form(items[b.second].P);
+        return fa != fb ? fa < fb : a.first > b.first;
     });
     sm_pe_batch* B = new (std::nothrow) sm_pe_batch();
     if (!B) return fail(SM_ERR_ALLOC, "host allocation failed");
@@ -264,16 +265,17 @@ int sm_pe_batch_create(sm_context* ctx, int n, const sm_geometry* const* geos, c
         B->host.push_back(b);
     }
     B->total = at;
-    // chunks of at most kBatchConst geometries, each with items from 0
-    for (size_t c0 = 0; c0 < B->host.size(); c0 += kBatchConst) {
-        const size_t c1 = std::min(B->host.size(), c0 + (size_t)kBatchConst);
+    // chunks of at most kBatchConst geometries of one form, each with items from 0
+    for (size_t c0 = 0, c1; c0 < B->host.size(); c0 = c1) {
+        const int form = pe_batch_form(B->host[c0].P);
+        for (c1 = c0 + 1; c1 < B->host.size() && c1 - c0 < (size_t)kBatchConst && pe_batch_form(B->host[c1].P) == form;) ++c1;
         const long long base = B->host[c0].tile_begin;
         long long end = base;
         for (size_t i = c0; i < c1; ++i) {
             B->host[i].tile_begin -= base;
             end = base + B->host[i].tile_begin + B->host[i].P.n_tiles;
         }
-        B->chunks.push_back({(int)c0, (int)(c1 - c0), end - base});
+        B->chunks.push_back({(int)c0, (int)(c1 - c0), form, end - base});
     }
     B->grid = ctx->sm_count * pe_batch_blocks_per_sm();
     int rc = check_cuda(cudaMalloc(&B->d_geoms, sizeof(PeBatchGeom) * B->host.size()), "batch table");
@@ -306,7 +308,7 @@ int sm_pe_batch_run(sm_pe_batch* b, void* stream_ptr) {
         cudaError_t e2 = cudaSuccess;
         for (const auto& c : b->chunks) {
             if (e2 == cudaSuccess)
-                e2 = pe_batch_launch(static_cast<const PeBatchGeom*>(b->d_geoms) + c.first, c.count, c.items,
+                e2 = pe_batch_launch(static_cast<const PeBatchGeom*>(b->d_geoms) + c.first, c.count, c.form, c.items,
                                      b->d_counter, b->grid, b->capture);
         }
         cudaError_t e3 = cudaStreamEndCapture(b->capture, &b->graph);

@@ -23,8 +23,8 @@
 //     does not cross contributes nothing either way, so the cone test is taken
 //     per ray and only for candidates with a nonzero chord (a float filter
 //     decides clear cases; cases within 1e-5 of the threshold use the
-//     reference's exact single-precision expression).  Each sub-point's own
-//     cone parameters are computed once per group of sub-points.
+//     reference's exact single-precision expression).  Candidates that pass it
+//     from every point of the voxel are flagged in the list and skip it.
 //  3. Lanes trace one ray (sub-point, sub-cell) each.  The rays of a group of
 //     sub-points are ordered (sub-cell column, sub-point, depth sub-cell) and
 //     dealt 32 to a warp pass, so a pass holds rays that run almost together
@@ -32,17 +32,22 @@
 //     cells seen from neighbouring sub-points): the lanes meet the same
 //     candidates and take the same branches.  Each pass first narrows the
 //     candidates to those its bundle of rays can reach (window test from the
-//     voxel's sub-point box to the box of the pass's sub-cell centres).  Per
-//     ray a division-free window test skips the exact test for candidates
-//     the ray cannot reach; the exact tests are the reference's
-//     single-precision ones, so every hit decision is the reference's.
-//     Skipped candidates would have contributed exactly 0.  The plates use a
-//     fast path that proves "fully traversed" with margins, else the exact
-//     test.  Values that are not hit decisions (solid angle, path inside the
-//     detecting crystal, absorption chord) use closed forms in single
-//     precision.
+//     voxel's sub-point box to the box of the pass's sub-cell centres), once
+//     for all groups of the voxel.  Per ray, division-free filters (chord_quick,
+//     chord_filter, hole_filter) call a candidate crossed, not crossed or
+//     unclear, with margins above the rounding of either form; unclear ones
+//     take the reference's single-precision test, so every hit decision is the
+//     reference's.  The plates are proved "fully traversed" with margins, per
+//     brick or per ray, else tested exactly.  Values that are not hit
+//     decisions (chords called by a filter, solid angle, path inside the
+//     detecting crystal, absorption chord) use closed forms in single precision.
 //  4. Lanes accumulate with Kahan summation; warp shuffles reduce; the CTA
 //     stages its 8 x brick results in shared memory and writes them out.
+//
+// What bounds it: 27.7 G warp instructions for 200 crystals x 4096 voxels of 64
+// x 16 rays behind two plates went out in 43 ms, 58 % of the issue slots; the
+// rest are fixed latencies of dependent instructions with 16 warps per SM
+// (128 registers and 113 KB of shared memory per CTA of 8).  DRAM is idle.
 #include <cuda_runtime.h>
 
 #include "pe.h"
@@ -1276,6 +1281,10 @@ __constant__ PeBatchGeom c_batch[kBatchConst];
 // geometries: each CTA takes the next item from a global counter until all
 // are done.  Geometries are laid out largest first, so the dynamic hand-out
 // balances the tail.  No CTA waits on another: the counter only hands out work.
+// The chunk's geometries are of one form (rays per entry, rotated crystals): all four
+// forms in one kernel took 244 bytes of spills and ran a sweep of 64 geometries 5 %
+// slower than a launch per geometry.
+template <bool FEW, bool ROT>
 __global__ void __launch_bounds__(kPeThreads, 2) pe_batch_kernel(int n_geoms, long long total,
                                                                  unsigned long long* counter) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1299,14 +1308,7 @@ __global__ void __launch_bounds__(kPeThreads, 2) pe_batch_kernel(int n_geoms, lo
         const int g = s_geom;
         if (item >= total) break;
         const PeBatchGeom& it = c_batch[g];
-        const long long tile = item - it.tile_begin;
-        if (it.P.pair > 1) {
-            if (it.P.rotated) pe_tile<false, true, true, false>(it.P, it.G, S, tile);
-            else pe_tile<false, true, false, false>(it.P, it.G, S, tile);
-        } else {
-            if (it.P.rotated) pe_tile<false, false, true, false>(it.P, it.G, S, tile);
-            else pe_tile<false, false, false, false>(it.P, it.G, S, tile);
-        }
+        pe_tile<false, FEW, ROT, false>(it.P, it.G, S, item - it.tile_begin);
         __syncthreads();
     }
 }
@@ -1318,7 +1320,7 @@ size_t pe_smem_bytes() { return sizeof(PeSmem); }
 // The dynamic shared memory limit is a per-device function attribute: set it
 // once per (device, kernel).
 static cudaError_t allow_smem(const void* fn, int which) {
-    static unsigned long long done[8] = {};
+    static unsigned long long done[11] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1352,25 +1354,31 @@ cudaError_t pe_launch(const PEParams& p, const DevGeometry& geo, bool record, lo
     return cudaGetLastError();
 }
 
-cudaError_t pe_batch_launch(const PeBatchGeom* geoms, int n_geoms, long long total, unsigned long long* counter,
-                            int grid, cudaStream_t stream) {
+int pe_batch_form(const PEParams& p) { return (p.pair > 1 ? 1 : 0) + (p.rotated ? 2 : 0); }
+
+cudaError_t pe_batch_launch(const PeBatchGeom* geoms, int n_geoms, int form, long long total,
+                            unsigned long long* counter, int grid, cudaStream_t stream) {
     if (total <= 0) return cudaSuccess;
     if (n_geoms < 1 || n_geoms > kBatchConst) return cudaErrorInvalidValue;
-    cudaError_t e = allow_smem((const void*)pe_batch_kernel, 7);
+    auto* const kernel = form == 0   ? pe_batch_kernel<false, false>
+                         : form == 1 ? pe_batch_kernel<true, false>
+                         : form == 2 ? pe_batch_kernel<false, true>
+                                     : pe_batch_kernel<true, true>;
+    cudaError_t e = allow_smem((const void*)kernel, 7 + form);
     if (e != cudaSuccess) return e;
     e = cudaMemcpyToSymbolAsync(c_batch, geoms, sizeof(PeBatchGeom) * (size_t)n_geoms, 0, cudaMemcpyDeviceToDevice,
                                 stream);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
-    pe_batch_kernel<<<grid, kPeThreads, sizeof(PeSmem), stream>>>(n_geoms, total, counter);
+    kernel<<<grid, kPeThreads, sizeof(PeSmem), stream>>>(n_geoms, total, counter);
     return cudaGetLastError();
 }
 
 int pe_batch_blocks_per_sm() {
     int n = 0;
-    if (allow_smem((const void*)pe_batch_kernel, 7) != cudaSuccess) return 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pe_batch_kernel, kPeThreads, sizeof(PeSmem)) != cudaSuccess)
+    if (allow_smem((const void*)pe_batch_kernel<false, false>, 7) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, pe_batch_kernel<false, false>, kPeThreads, sizeof(PeSmem)) != cudaSuccess)
         return 1;
     return n > 0 ? n : 1;
 }

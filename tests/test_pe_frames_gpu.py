@@ -5,6 +5,7 @@ reference's single-precision decisions and double magnitudes: no decision differ
 error is that of single-precision arithmetic, 1e-4 as for the kernel's other tests."""
 import numpy as np
 import pytest
+import torch
 
 import oracle_py
 import sysmat_b200
@@ -34,4 +35,28 @@ def test_frames_and_candidate_counts(layers, sv, sc, rotated):
     assert np.allclose(g.pe(), A, rtol=1e-4, atol=1e-30)
     assert ctx.last_counters()[0] == p.n_crystals * p.n_voxels * np.prod(sv) * np.prod(sc)
     g.close()
+    ctx.close()
+
+
+def test_a_batch_of_all_forms_equals_single_launches():
+    """Rotated and unrotated detectors, few and many rays per entry, in one batch (a launch per form)."""
+    ctx = sysmat_b200.Context(0)
+    geos, opts, single = [], [], []
+    for i in range(8):
+        p = configs.tiny(seed=i, layers=1 + i % 3, rotated=bool(i & 1))
+        if i & 2:
+            p.sv = (2, 2, 2)
+        g = sysmat_b200.Geometry(ctx, p)
+        geos.append(g)
+        opts.append(g.options())
+        single.append(g.pe(opts=opts[-1]))
+    outs = [torch.zeros(a.shape, dtype=torch.float32, device="cuda") for a in single]
+    batch = sysmat_b200.PeBatch(ctx, geos, opts, [o.data_ptr() for o in outs], [o.shape[1] for o in outs])
+    batch.run()
+    torch.cuda.synchronize()
+    for a, o in zip(single, outs):
+        assert np.allclose(o.cpu().numpy(), a, rtol=1e-4, atol=1e-30)
+    batch.close()
+    for g in geos:
+        g.close()
     ctx.close()
