@@ -361,7 +361,8 @@ def run_ours(args, world, rank, local):
     entries_per_step = rows * slab_vox
     value = world * args.steps * entries_per_step / (total_ms / 1e3)
 
-    # Work counters of one slab (separate, counted run).
+    # Work counters of one slab (separate, counted run): crystals and holes whose chord the
+    # rays took, i.e. crossed ones and the few that the filters leave to the exact test.
     ctx.set_counters(True)
     geo.pe(z=(0, SLAB_Z), rows=row_range, opts=opts, out=out.data_ptr(), stream=stream.cuda_stream)
     n_rays, n_cry, n_hole, n_cone = ctx.last_counters()

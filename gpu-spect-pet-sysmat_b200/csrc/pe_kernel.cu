@@ -44,8 +44,8 @@
 //  4. Lanes accumulate with Kahan summation; warp shuffles reduce; the CTA
 //     stages its 8 x brick results in shared memory and writes them out.
 //
-// What bounds it: 27.7 G warp instructions for 200 crystals x 4096 voxels of 64
-// x 16 rays behind two plates went out in 43 ms, 58 % of the issue slots; the
+// What bounds it: 26.2 G warp instructions for 200 crystals x 16384 voxels of 64
+// x 16 rays behind two plates go out in 36 ms, 64 % of the issue slots; the
 // rest are fixed latencies of dependent instructions with 16 warps per SM
 // (128 registers and 113 KB of shared memory per CTA of 8).  DRAM is idle.
 #include <cuda_runtime.h>

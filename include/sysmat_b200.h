@@ -170,9 +170,10 @@ int sm_pe_record_hits(sm_context* ctx, const sm_geometry* geo, const sm_pe_optio
                       int32_t* out, int* record_words);
 
 /* Work counters: when enabled, each sm_pe_compute on the context counts rays
- * traced, exact crystal tests, exact hole tests and candidate cone tests
- * (the cone test is taken on the candidates a ray crosses) (costs a little
- * time and synchronises the call). */
+ * traced, crystals and holes whose chord a ray took (those its filters called
+ * crossed, or left to the exact test) and candidate cone tests (taken on
+ * crossed candidates that do not pass for the whole voxel).  Costs a few per
+ * cent of the time and synchronises the call. */
 int sm_pe_set_counters(sm_context* ctx, int enable);
 int sm_pe_last_counters(sm_context* ctx, int64_t out[4]);
 
