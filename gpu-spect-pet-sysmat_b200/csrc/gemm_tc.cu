@@ -28,8 +28,9 @@
 //
 // Every wait is bounded (wait_limit polls, set process-wide by
 // sm_tc_wait_limit): a wait that runs out sets the error word, the roles stop and
-// skip their epilogue; copies and MMAs still in flight are then waited for
-// (bounded by the default limit), and the CTA frees its TMEM and returns.
+// skip their epilogue.  Any role may be the one that fails, so only once all have
+// stopped are the copies and MMAs still in flight waited for (bounded by the default
+// limit); then the CTA frees its TMEM and returns.
 #include <atomic>
 #include <cstdint>
 
@@ -251,9 +252,9 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
         return false;
     };
 
+    uint32_t it = 0, keeps = 0;   // this role's chunks and kept B tiles so far
     if (warp == kWarpTma) {
         if ((TA || TB) && lane == 0) {
-            uint32_t it = 0, keeps = 0;
             int kept_n = -1;
             bool ok = true;
             for (Walk<BN> at(g); at.more && ok; at.next()) {
@@ -272,15 +273,11 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
                     if (TB && !KEEP) tma_load(S.b[s], &map_b, c * kChunkK, at.n0(), &S.landed[s]);
                 }
             }
-            if (*failed && keeps) mbar_wait(&S.kept, (keeps - 1) & 1u, kWaitLimit);
-            if (*failed)   // copies in flight land before the CTA goes
-                for (uint32_t i = it < (uint32_t)R::kStages ? 0u : it - R::kStages; i < it; ++i)
-                    mbar_wait(&S.landed[i % R::kStages], (i / R::kStages) & 1u, kWaitLimit);
         }
     } else if (warp == kWarpMma) {
         if (lane == 0) {
             const uint32_t idesc = instr_desc(BN);
-            uint32_t it = 0, n = 0, keeps = 0;
+            uint32_t n = 0;
             int kept_n = -1;
             bool ok = true;
             for (Walk<BN> at(g); at.more && ok; ++n) {
@@ -315,10 +312,6 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
                 if (ok) commit(&S.acc_full[n & 1u]);
                 at.next();
                 if (KEEP && ok && at.more && at.n0() != kept_n) commit(&S.unkept);
-            }
-            if (*failed) {   // MMAs in flight finish before the tensor memory goes
-                commit(&S.drain);
-                mbar_wait(&S.drain, 0, kWaitLimit);
             }
         }
     } else if (warp < kWarpLoad) {
@@ -391,7 +384,6 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
             if (lane == 0) arrive(&S.acc_empty[n & 1u]);
         }
     } else if (!(TA && TB)) {
-        uint32_t it = 0;
         bool ok = true;
         for (Walk<BN> at(g); at.more && ok; at.next()) {
             for (int c = 0; c < chunks; ++c, ++it) {
@@ -409,7 +401,20 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (threadIdx.x == 0 && *failed && g.error) atomicOr(g.error, 1);
+    if (*failed) {   // no role sets it any more, so all take this branch or none
+        if (threadIdx.x == 0 && g.error) atomicOr(g.error, 1);
+        if (warp == kWarpTma && lane == 0) {   // copies land before the CTA goes
+            if (keeps) mbar_wait(&S.kept, (keeps - 1) & 1u, kWaitLimit);
+            for (uint32_t i = it < (uint32_t)R::kStages ? 0u : it - R::kStages; i < it; ++i)
+                mbar_wait(&S.landed[i % R::kStages], (i / R::kStages) & 1u, kWaitLimit);
+        }
+        if (warp == kWarpMma && lane == 0) {   // MMAs finish before the tensor memory goes
+            commit(&S.drain);
+            mbar_wait(&S.drain, 0, kWaitLimit);
+        }
+        __syncwarp();
+        __syncthreads();
+    }
     if (warp == kWarpMma) {
         asm volatile("tcgen05.fence::after_thread_sync;");
         tmem_dealloc(tmem, 2 * BN);

@@ -302,8 +302,8 @@ int sm_gemm_bf16(int m, int n, int k, const void* a, int64_t a_ms, int64_t a_ks,
 
 /* The bound on every wait of sm_gemm_bf16 (and of the surrogate network's
  * GEMMs) for its own MMAs: mbarrier polls before the kernel gives up, sets
- * *error, skips its epilogue, waits (bounded by the default) for MMAs still in
- * flight, frees its tensor memory and returns.  Process-wide; applies to
+ * *error, skips its epilogue, waits (bounded by the default) for copies and MMAs
+ * still in flight, frees its tensor memory and returns.  Process-wide; applies to
  * launches after the call.  polls < 0 restores the default (2^26); 0 makes
  * every wait give up at once (for testing the error path).  previous (may be
  * NULL) receives the limit in force before. */
