@@ -52,8 +52,11 @@ __device__ __forceinline__ float row_threshold(float mx, float frac) {
     return mx > 0.0f ? __fmul_rn(frac, mx) : 1.0f;
 }
 
-// Longest row beam_fused_kernel takes: two copies of it and the counts in 227 KB.
+// Longest row beam_fused_kernel takes: two copies of it and the counts in 227 KB, of which
+// the block's own variables take 1 KB.
 constexpr int kFusedVoxels = 23000;
+constexpr int kFusedBytes = 226 * 1024;
+static_assert(sizeof(float) * kFusedVoxels * 5 / 2 <= kFusedBytes, "two copies and the counts fit");
 
 __device__ __forceinline__ void copy_async(float* dst, const float* src, bool wide) {
     const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
@@ -191,6 +194,7 @@ __global__ void __launch_bounds__(1024) beam_fused_kernel(const float* __restric
 // the chain of its reductions) and 171 us for the two passes over global memory.
 constexpr int kHeldThreads = 512, kHeld = 8;   // float4 per thread
 constexpr int kHeldVoxels = kHeldThreads * 4 * kHeld;
+constexpr int kHeldBytes = sizeof(float) * kHeldVoxels + 16;
 
 __global__ void __launch_bounds__(kHeldThreads, 2) beam_held_kernel(const float* __restrict__ A, long long rows, int V, long long ld,
                                                           float frac, float* __restrict__ row_max,
@@ -470,14 +474,16 @@ extern "C" int sm_beam_metrics(const float* sysmat, int64_t rows, int64_t voxels
         // three rows of shared memory where they fit, else two
         int threads = 32;
         while (threads < 1024 && threads * (V < 2048 ? 16 : 32) < V) threads *= 2;
-        const int stages = 3 * row + row / 2 + 1024 <= 226 * 1024 ? 3 : 2;
+        const int stages = 3 * row + row / 2 + 1024 <= kFusedBytes ? 3 : 2;
         size_t smem = stages * row + row / 2;
         if (held) {
             threads = kHeldThreads;
             smem = row + 16;
         }
-        auto launch = [&](auto kernel) -> cudaError_t {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // `most`: the kernel's largest row.  The attribute is the kernel's, not the launch's: a
+        // value of this call's own would fail the launch of a thread with longer rows.
+        auto launch = [&](auto kernel, int most) -> cudaError_t {
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
             int per_sm = 0;
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
             if (e != cudaSuccess) return e;
@@ -490,9 +496,9 @@ extern "C" int sm_beam_metrics(const float* sysmat, int64_t rows, int64_t voxels
                                                               ld_mask, out);
             return cudaGetLastError();
         };
-        if (held) SM_CUDA(launch(beam_held_kernel));
-        else SM_CUDA(vec ? (stages == 3 ? launch(beam_fused_kernel<true, 3>) : launch(beam_fused_kernel<true, 2>))
-                    : (stages == 3 ? launch(beam_fused_kernel<false, 3>) : launch(beam_fused_kernel<false, 2>)));
+        if (held) SM_CUDA(launch(beam_held_kernel, kHeldBytes));
+        else SM_CUDA(vec ? (stages == 3 ? launch(beam_fused_kernel<true, 3>, kFusedBytes) : launch(beam_fused_kernel<true, 2>, kFusedBytes))
+                    : (stages == 3 ? launch(beam_fused_kernel<false, 3>, kFusedBytes) : launch(beam_fused_kernel<false, 2>, kFusedBytes)));
         return SM_OK;
     }
     const long long grid1 = rows < (long long)sms * 8 ? rows : (long long)sms * 8;
