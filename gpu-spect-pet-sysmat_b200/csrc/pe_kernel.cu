@@ -1274,7 +1274,8 @@ __global__ void __launch_bounds__(kPeThreads, 2) pe_trace_kernel(const __grid_co
 // The batch's geometries, in constant memory: the tile code reads launch
 // parameters in its inner loops, and constant-bank loads of a warp-uniform
 // index cost what kernel-parameter loads cost.  Written by the batch's own
-// graph (a device-to-device copy before each chunk's launch).
+// graph (a device-to-device copy before each chunk's launch); sm_pe_batch_run keeps
+// the runs of a device in order.
 __constant__ PeBatchGeom c_batch[kBatchConst];
 
 // Persistent kernel over the (geometry, tile) items of up to kBatchConst

@@ -202,7 +202,8 @@ int sm_pe_batch_create(sm_context* ctx, int n, const sm_geometry* const* geos, c
 int sm_pe_batch_info(const sm_pe_batch* batch, int64_t out[3]);
 /* One launch of the batch on `stream` (asynchronous; sm_context_sync reports
  * device-side capacity errors).  The first call captures the launch in a
- * CUDA graph; later calls replay it. */
+ * CUDA graph; later calls replay it.  Runs on one device, of any batches and
+ * streams, follow each other. */
 int sm_pe_batch_run(sm_pe_batch* batch, void* stream);
 int sm_pe_batch_destroy(sm_pe_batch* batch);
 
