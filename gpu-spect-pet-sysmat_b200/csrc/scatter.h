@@ -47,7 +47,7 @@ struct ScatterTables {
     const float4* hole_src;      // layer-0 hole scatter point x, (y1 + y2) / 2 + Image[11], z, y2 - y1
     const float4* crystal_src;   // scatter points of every crystal, [crystal][point]: world x, y, z, 0
     const KnNode* kn;            // kKnNodes + 1 nodes
-    const float4* erfc;          // kErfcNodes nodes (scatter_term.cuh)
+    const float4* window;        // kWindowNodes nodes (scatter_term.cuh)
     int n_crystals;
     int n_holes0;                // holes of plate 0 (Collimator[10])
     int n_points;                // scatter points per crystal
@@ -100,7 +100,7 @@ struct ScatterParams {
 struct HostScatterTables {
     std::vector<float> crystal_raw, hole_raw, hole_src, crystal_src;
     std::vector<KnNode> kn;
-    std::vector<float4> erfc;
+    std::vector<float4> window;
     int n_points = 1;
     int sp[3] = {1, 1, 1};
     float chord_delta = 0.0f;

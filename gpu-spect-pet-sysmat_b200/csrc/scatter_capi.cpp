@@ -25,17 +25,17 @@ int upload_tables(const HostScatterTables& H, int n_crystals, int n_holes0, cuda
                   ScatterTables* T) {
     const size_t b_raw = H.crystal_raw.size() * 4, b_hraw = H.hole_raw.size() * 4, b_hsrc = H.hole_src.size() * 4,
                  b_src = H.crystal_src.size() * 4, b_kn = H.kn.size() * sizeof(KnNode),
-                 b_erfc = H.erfc.size() * sizeof(float4);
+                 b_win = H.window.size() * sizeof(float4);
     auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t o_raw = 0, o_hraw = up(b_raw), o_hsrc = o_hraw + up(b_hraw), o_src = o_hsrc + up(b_hsrc),
-                 o_kn = o_src + up(b_src), o_erfc = o_kn + up(b_kn), total = o_erfc + up(b_erfc);
+                 o_kn = o_src + up(b_src), o_win = o_kn + up(b_kn), total = o_win + up(b_win);
     std::vector<unsigned char> host(total, 0);
     std::memcpy(host.data() + o_raw, H.crystal_raw.data(), b_raw);
     std::memcpy(host.data() + o_hraw, H.hole_raw.data(), b_hraw);
     std::memcpy(host.data() + o_hsrc, H.hole_src.data(), b_hsrc);
     std::memcpy(host.data() + o_src, H.crystal_src.data(), b_src);
     std::memcpy(host.data() + o_kn, H.kn.data(), b_kn);
-    std::memcpy(host.data() + o_erfc, H.erfc.data(), b_erfc);
+    std::memcpy(host.data() + o_win, H.window.data(), b_win);
     SM_TRY(blob->alloc(total, s, "scatter tables"));
     SM_CUDA(cudaMemcpyAsync(blob->p, host.data(), total, cudaMemcpyHostToDevice, s));
     SM_CUDA(cudaStreamSynchronize(s));   // the staging buffer is released on return
@@ -45,7 +45,7 @@ int upload_tables(const HostScatterTables& H, int n_crystals, int n_holes0, cuda
     T->hole_src = reinterpret_cast<const float4*>(b + o_hsrc);
     T->crystal_src = reinterpret_cast<const float4*>(b + o_src);
     T->kn = reinterpret_cast<const KnNode*>(b + o_kn);
-    T->erfc = reinterpret_cast<const float4*>(b + o_erfc);
+    T->window = reinterpret_cast<const float4*>(b + o_win);
     T->n_crystals = n_crystals;
     T->n_holes0 = n_holes0;
     T->n_points = H.n_points;

@@ -196,8 +196,8 @@ int build_scatter_tables(const HostGeometry& g, const int sp[3], HostScatterTabl
     for (int a = 0; a < 3; ++a) s2 += (hi[a] - lo[a]) * (hi[a] - lo[a]);
     T.chord_delta = 1.5e-6f * std::sqrt(s2);
     build_kn_table(g.physics[7], &T.kn, &T.kn_inv_norm);
-    T.erfc.resize(kErfcNodes);
-    build_erfc_table(T.erfc.data());
+    T.window.resize(kWindowNodes);
+    build_window_table(T.window.data());
     return SM_OK;
 }
 

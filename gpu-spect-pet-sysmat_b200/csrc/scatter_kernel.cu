@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(kScThreads, 2) scatter_main_kernel(const __gri
                 const float isx = (V.x - D.x) * D.cm - (V.z - D.z) * D.sm;
                 const float isy = V.y - D.y;
                 const float isz = (V.x - D.x) * D.sm + (V.z - D.z) * D.cm;
-                const float t = scatter_term<true>(P, D, c, S.kn, T.erfc, T.kn_inv_norm, V.x, V.y, V.z, isx, isy, isz);
+                const float t = scatter_term<true>(P, D, c, S.kn, T.window, T.kn_inv_norm, V.x, V.y, V.z, isx, isy, isz);
                 add = (double)(S.wgt[slot][col][j] * t);
             }
             // a cell may wait for several points: one point at a time
