@@ -164,22 +164,30 @@ SM_HD void angle_parts(float ux, float uy, float uz, const float3& e, float* sin
     *cosine = fmaf(ux, e.x, fmaf(uy, e.y, uz * e.z));
 }
 
-// atan2(s, c) for s >= 0 to 3e-7: a least-maximum polynomial of atan(t) / t in t^2
-// (relative error 1.5e-8, fitted for this file) on the smaller quotient.
+// atan2(s, c) for s >= 0: atan(t) = t + t x q(x), x = t^2, of the smaller quotient t <= 1.
+// q fits the relative error of the whole in the least-maximum sense (Lawson's reweighted
+// least squares on 4001 Chebyshev points; each coefficient rounded to a float in turn, from
+// the highest, and the rest fitted again): 2.3e-8 with the coefficients as written.  The
+// quotient is corrected once and pi / 2 and pi are carried to more than 24 bits, so the
+// rest is rounding.  (Not FINE, for a decision with a margin: without these two, to 3e-7.)  On the GPU 3e-8 rad in the mean square for angles to 0.8, 8e-8 to pi;
+// atan2f, which it stands for, 3e-8 and 1.1e-7.
+template <bool FINE = true>
 SM_HD float angle_quick(float s, float c) {
     const float a = fabsf(c), lo = fminf(s, a), hi = fmaxf(s, a);
-    const float t = hi > 0.0f ? sm_fdiv(lo, hi) : 0.0f, x = t * t;
-    float p = 0.00284988945f;
-    p = fmaf(p, x, -0.0160686299f);
-    p = fmaf(p, x, 0.0426915251f);
-    p = fmaf(p, x, -0.0750429556f);
-    p = fmaf(p, x, 0.106409349f);
-    p = fmaf(p, x, -0.142036453f);
-    p = fmaf(p, x, 0.199926198f);
-    p = fmaf(p, x, -0.333330721f);
-    p = fmaf(p, x, 1.0f) * t;
-    if (s > a) p = 1.57079632679489662f - p;
-    return c < 0.0f ? 3.14159265358979324f - p : p;
+    const float t = !(hi > 0.0f) ? 0.0f : (FINE ? near_div(lo, hi, fast_rcp(hi)) : sm_fdiv(lo, hi)), x = t * t;
+    float q = 0.00292069255f;
+    q = fmaf(q, x, -0.0163679291f);
+    q = fmaf(q, x, 0.0432118624f);
+    q = fmaf(q, x, -0.0755221471f);
+    q = fmaf(q, x, 0.106660053f);
+    q = fmaf(q, x, -0.142110556f);
+    q = fmaf(q, x, 0.199937731f);
+    q = fmaf(q, x, -0.333331525f);
+    float p = fmaf(t * x, q, t);
+    const bool steep = s > a, back = c < 0.0f;
+    const float turn = steep ? 1.57079632679489662f : (back ? 3.14159265358979324f : 0.0f);
+    if (steep != back) p = -p;
+    return turn + (FINE ? fmaf(turn, -2.78275e-8f, p) : p);   // pi's float is above pi by 2.78275e-8 of it
 }
 
 // Polar range of the unit seen from S along u: the lowest angle and the reference's
@@ -200,7 +208,7 @@ SM_HD PolarRange polar_range(float ux, float uy, float uz, const float3& near, c
     float steps = 0.0f;
     if (QUICK) {
         r.lo = from_zero ? 0.0f : angle_quick(sn, cn);
-        steps = (angle_quick(sf, cf) - r.lo) * 100.0f;
+        steps = (angle_quick<false>(sf, cf) - r.lo) * 100.0f;
         r.n = (int)steps;
     }
     if (!QUICK || fabsf(steps - rintf(steps)) < 2e-4f) {
@@ -321,8 +329,8 @@ SM_HD void make_src(const Det& D, float4 S, float4 pr, Src& C) {
 // One term without its weight W.  I: voxel (world); Is: voxel in the detector
 // frame.  SrcT: Src, or a view of one kept in shared memory (same members).
 // QUICK: the window probability from a table and the polar range from quick
-// angles (a seventh less work, values within 1e-7); the transfer matrices, which
-// are rounded to bf16 and compared with the exact columns at a thousandth of their
+// angles (a seventh less work, errors no larger); the transfer matrices, which are
+// rounded to bf16 and compared with the exact columns at a thousandth of their
 // size, keep the other form.
 template <bool QUICK, class SrcT>
 SM_HD float scatter_term(const ScatterParams& P, const Det& D, const SrcT& C, const KnNode* kn, const float4* window_nodes,
