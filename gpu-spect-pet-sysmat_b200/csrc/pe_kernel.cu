@@ -512,6 +512,12 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
         const float through = pb.thickness * r * fast_rcp(dy);   // T / cos(theta)
         if ((through - in_holes) >= 0.00001f) att += pb.mu_total * (through - in_holes);
     }
+    auto note = [&](int k, float len) {           // a crystal of the hit record
+        if (!RECORD || !(len > 0.0f)) return;
+        if (rec_c < kRecCrystals) rec[3 + kRecHoles + rec_c] = S.c_id[k];
+        else atomicOr(status, kStatusRecordOverflow);
+        ++rec_c;
+    };
     // Other crystals among the candidates, each in its own frame (:687-725).
     // `f` and `len`: chord_quick's call in the world's frame, -1 for a rotated crystal.
     auto settle = [&](int e, const float4& kp, const float4& kh, int f, float len) {
@@ -558,17 +564,13 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             if (!g) return;
         }
         att += len * kp.w;
-        if (RECORD && len > 0.0f) {
-            if (rec_c < kRecCrystals) rec[3 + kRecHoles + rec_c] = S.c_id[k];
-            else atomicOr(status, kStatusRecordOverflow);
-            ++rec_c;
-        }
+        note(k, len);
     };
     const int nwc = (L.n_c + 31) >> 5;
     for (int wd = 0; wd < nwc; ++wd) {
         unsigned bits = L.pass_c[wd];
         while (bits) {
-            if (FEW || ROT || RECORD) {
+            if (FEW || ROT) {
                 const int b = __ffs(bits) - 1;
                 bits &= bits - 1;
                 const int e = L.list_c[(wd << 5) + b], k = e & kIndex;
@@ -599,6 +601,8 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             if ((f0 | f1) > 0 && !(f0 && !(e0 & kConeSure)) && !(f1 && !(e1 & kConeSure))) {
                 if (f0) att += len0 * kp0.w;
                 if (f1) att += len1 * kp1.w;
+                if (RECORD && f0) note(e0 & kIndex, len0);
+                if (RECORD && f1) note(e1 & kIndex, len1);
                 if (COUNT) n.crystal += f0 + f1;
                 continue;
             }
@@ -991,12 +995,14 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                 hiy = __reduce_max_sync(0xffffffffu, in ? iy : -1);
                 hiz = __reduce_max_sync(0xffffffffu, in ? iz : -1);
             }
-            int rec_slot = -1;
+            int rec_slot = -1;                     // of this lane's voxel
+            unsigned traced = valid;               // the group's voxels to trace: all, or the recorded
             if (RECORD) {
                 const long long vox = ((long long)iz * P.ny + iy) * P.nx + ix;
                 for (int i = 0; i < P.rec_n; ++i)
                     if (P.rec_rows[i] == d && P.rec_vox[i] == vox) rec_slot = i;
-                if (rec_slot < 0) continue;
+                traced = __ballot_sync(0xffffffffu, in && rec_slot >= 0) & 0xffu;
+                if (!traced) continue;
             }
             float acc = 0.0f, comp = 0.0f;
             int lane_vox = VP == 1 ? 0 : fast_div(lane, span ? span : 32, span ? inv_span : 0.03125f);
@@ -1067,10 +1073,11 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                     // The candidates do not fit the shared-memory lists: the group's
                     // voxels through the geometry tables, same decisions and values.
                     for (int u = 0; u < VP; ++u) {
-                        if (!((valid >> u) & 1u)) continue;
+                        if (!((traced >> u) & 1u)) continue;
                         int x, y, z;
                         vox_of(u, x, y, z);
-                        const float w = slow_voxel<RECORD>(P, G, S, D, d, x, y, z, rec_slot, lane);
+                        const int slot = RECORD ? __shfl_sync(0xffffffffu, rec_slot, u) : -1;
+                        const float w = slow_voxel<RECORD>(P, G, S, D, d, x, y, z, slot, lane);
                         if (lane == 0) S.out[warp][vl + u] = w * P.inv_sv;
                     }
                     __syncwarp();
@@ -1188,8 +1195,9 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                                 p = Vec3{p4.x, p4.y, p4.z};
                                 csp = &L.cs[j];
                                 if (has) lane_vox = __float_as_int(p4.w);
-                                active = has && ((valid >> lane_vox) & 1u);
+                                active = has && ((traced >> lane_vox) & 1u);
                             }
+                            const int slot = RECORD ? __shfl_sync(0xffffffffu, rec_slot, FEW ? lane_vox : 0) : -1;
                             if (active) {
                                 if (!FEW) p = subpoint_of(P, ix, iy, iz, s0 + j);
                                 // ... in the detecting crystal's frame
@@ -1198,8 +1206,8 @@ __device__ __forceinline__ void pe_tile(const PEParams& P, const DevGeometry& G,
                                 int* rec = nullptr;
                                 if (RECORD) {
                                     const int c = (sz * P.dX + sx) * P.dY + sy;   // the oracle's sub-cell order
-                                    rec = P.rec_out + ((long long)rec_slot * P.n_sv * P.n_sc + (long long)(s0 + j) * P.n_sc + c) *
-                                                          kRecWords;
+                                    const int pt = s0 + j - (FEW ? lane_vox * P.n_sv : 0);   // of its voxel
+                                    rec = P.rec_out + ((long long)slot * P.n_sv * P.n_sc + (long long)pt * P.n_sc + c) * kRecWords;
                                 }
                                 const float v = trace_ray<RECORD, FEW, ROT, COUNT>(P, G, S, L, plates_sure, any_hole, csp, D, p, ps, cell, rec,
                                                                   P.status, counts);
@@ -1321,7 +1329,7 @@ size_t pe_smem_bytes() { return sizeof(PeSmem); }
 // The dynamic shared memory limit is a per-device function attribute: set it
 // once per (device, kernel).
 static cudaError_t allow_smem(const void* fn, int which) {
-    static unsigned long long done[11] = {};
+    static unsigned long long done[14] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1343,8 +1351,12 @@ cudaError_t pe_launch(const PEParams& p, const DevGeometry& geo, bool record, lo
     // Counting instantiations of their own: the counters take 14 registers of the loop.
     // Detectors without a rotated crystal, the usual ones, leave the frames' code out: a
     // sweep of 40 entries of 16 rays 319 -> 288 ms, 64-ray entries 8.3 -> 7.5 ms.
+    // Hit records are traced by the forms that the matrix takes.
     cudaError_t e;
-    if (record) e = launch(pe_trace_kernel<true, false, true, false>, 0);
+    if (record && p.rotated)
+        e = p.pair > 1 ? launch(pe_trace_kernel<true, true, true, false>, 0) : launch(pe_trace_kernel<true, false, true, false>, 11);
+    else if (record)
+        e = p.pair > 1 ? launch(pe_trace_kernel<true, true, false, false>, 12) : launch(pe_trace_kernel<true, false, false, false>, 13);
     else if (p.counters)
         e = p.pair > 1 ? launch(pe_trace_kernel<false, true, true, true>, 1) : launch(pe_trace_kernel<false, false, true, true>, 2);
     else if (p.rotated)
