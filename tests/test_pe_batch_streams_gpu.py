@@ -1,4 +1,5 @@
-"""Two batches of other geometries at once, each on a stream of its own: every matrix equals,
+"""Two batches of other geometries at once, each on a stream of its own, between them all four
+forms (few or many rays per entry, without or with rotated crystals): every matrix equals,
 bit for bit, what the geometry gives alone."""
 import numpy as np
 import pytest
@@ -12,8 +13,11 @@ pytestmark = pytest.mark.gpu
 def test_batches_on_two_streams():
     import torch
     ctx = sysmat_b200.Context(0)
+    many_rotated = configs.tiny(seed=3, rotated=True)
+    many_rotated.sv = (2, 2, 2)
     sets = [[configs.tiny(seed=i, layers=1 + i % 3, rotated=i == 4) for i in range(5)],
-            [configs.two_plates_small(seed=8), configs.tiny(seed=9, layers=2), configs.sweep_small()[3]]]
+            [configs.two_plates_small(seed=8), configs.tiny(seed=9, layers=2), many_rotated,
+             configs.sweep_small()[3]]]
     geos = [[sysmat_b200.Geometry(ctx, p) for p in params] for params in sets]
     want = [[g.pe() for g in gs] for gs in geos]
     outs = [[torch.empty(w.shape, device="cuda") for w in ws] for ws in want]
