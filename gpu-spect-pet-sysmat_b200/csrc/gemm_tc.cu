@@ -122,7 +122,9 @@ __device__ __forceinline__ void load_rows(unsigned char* dst, int rows, const __
                                           long long ks, int r0, int rows_total, int k0, int k_total, int warp, int lane) {
     if (ks == 1) {
         // lane = two consecutive k of a row, eight rows in flight.  A row that starts off
-        // a 4-byte boundary is read one element early and shifted across the lanes.
+        // a 4-byte boundary is read one element early and shifted across the lanes; the word
+        // holds the row's first element too, so it lies in the operand's memory whatever the
+        // stride.
         const char* bytes = reinterpret_cast<const char*>(src);
         const unsigned base_off = (unsigned)(reinterpret_cast<uintptr_t>(src) >> 1) & 1u, odd = (unsigned)rs & 1u;
         const bool full = k0 + kChunkK <= k_total;
@@ -316,6 +318,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
         }
     } else if (warp < kWarpLoad) {
         const int part = warp & 3;                     // TMEM lanes 32 part .. 32 part + 31
+        static_assert(kStoreWarps == 4, "a store warp for each 32 TMEM lanes");
         float(*out)[36] = S.out[warp - kWarpStore];
         const bool vec = g.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(g.c) & 15u) == 0 &&
                          (!g.bias || (reinterpret_cast<uintptr_t>(g.bias) & 15u) == 0);
@@ -326,7 +329,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
             asm volatile("tcgen05.fence::after_thread_sync;");
             const float scale = g.row_scale && m0 + lane < g.m ? g.row_scale[m0 + lane] : g.alpha;
             const int cols = min(BN, g.n - n0);
-            for (int c0 = (warp - kWarpStore) / 4 * 32; c0 < cols; c0 += 32 * (kStoreWarps / 4)) {
+            for (int c0 = 0; c0 < cols; c0 += 32) {
                 float v[32];
                 tmem_load32(tmem + (n & 1u) * BN + ((uint32_t)(32 * part) << 16) + (uint32_t)c0, v);
 #pragma unroll
@@ -341,7 +344,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ GemmArgs g, const __grid_constant__ 
                 const long long step = 4 * g.ldc;
                 if (vec && m0 + 32 <= g.m && c0 + 32 <= cols) {
                     // a whole 32 x 32 block: no test per row, one warp per scheduler has nobody to hide it
-                    if (g.bias) {
+                    if (g.bias && g.epilogue != 1) {
                         const float4 o = __ldg(reinterpret_cast<const float4*>(g.bias + col));
 #pragma unroll
                         for (int i = 0; i < 8; ++i) w[i] = make_float4(w[i].x + o.x, w[i].y + o.y, w[i].z + o.z, w[i].w + o.w);
@@ -491,7 +494,6 @@ uint32_t gemm_wait_limit(int64_t polls) {
 
 cudaError_t gemm_bf16_tc(const GemmArgs& args, cudaStream_t stream) {
     if (args.m <= 0 || args.n <= 0 || args.k <= 0) return cudaSuccess;
-    if (args.n_tile != 64 && args.n_tile != 128 && args.n_tile != 256) return cudaErrorInvalidValue;
     int dev = 0, sms = 148;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -28,7 +28,6 @@ extern "C" int sm_gemm_bf16(int m, int n, int k, const void* a, int64_t a_ms, in
     g.row_scale = row_scale;
     g.bias = bias;
     g.accumulate = accumulate;
-    g.n_tile = n_tile;
     g.error = error;
     SM_CUDA(gemm_bf16_tc(g, (cudaStream_t)stream));
     return SM_OK;

@@ -34,7 +34,6 @@ namespace {
 constexpr int kEw = 256;
 
 int blocks_for(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + kEw - 1) / kEw, 148LL * 16)); }
-int n_tile_for(int n) { return n >= 192 ? 256 : (n > 64 ? 128 : 64); }
 
 // out [n][6F] and, when set, outT [6F][n]
 __global__ void fourier_kernel(const int* __restrict__ vox, int n, int nx, int ny, int nz, int F,
@@ -286,7 +285,6 @@ int SurrogateNet::gemm(int m, int n, int k, const __nv_bfloat16* a, int64_t ams,
     g.bias = bias;
     g.accumulate = 0;
     g.epilogue = epilogue;
-    g.n_tile = n_tile_for(n);
     g.error = error;
     SM_CUDA(gemm_bf16_tc(g, st));
     return SM_OK;
