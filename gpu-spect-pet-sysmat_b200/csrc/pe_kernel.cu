@@ -245,9 +245,12 @@ __device__ __forceinline__ Box3 box_of(const float4& lo, const float4& hi) {
 }
 
 // ---- division-free window test -------------------------------------------------
-// window_hit (tracer.cuh) with the bundle source A and target B fixed: the two
-// reciprocals are computed once.  Conservative: K carries the 0.01 mm margin,
-// far above the error of the approximate reciprocals.
+// Conservative culling: can any segment from a point of box A to a point of box B meet
+// box K?  Uses the depth (y) ordering of the scanner: at depth y a segment a -> b sits at
+// lateral position a + (b - a) * lambda, lambda = (y - a_y) / (b_y - a_y); lambda is
+// monotone in y, a_y and b_y, so its range over K's depth band comes from box corners.
+// True whenever the ordering assumption fails.  The two reciprocals are computed once per
+// bundle; K carries a 0.01 mm margin, far above the error of the approximate reciprocals.
 struct Bundle {
     Box3 A, B;
     float inv2;     // 1 / (B.y2 - A.y2)

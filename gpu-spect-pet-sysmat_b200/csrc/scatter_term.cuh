@@ -321,11 +321,6 @@ SM_HD float column_max_cos(const Src& C, float i0x, float i0y, float i0z, float 
     return m;
 }
 
-SM_HD void make_src(const Det& D, float4 S, float4 pr, Src& C) {
-    make_src_basic(D, S, C);
-    make_src_rest(D, pr, C);
-}
-
 // One term without its weight W.  I: voxel (world); Is: voxel in the detector
 // frame.  SrcT: Src, or a view of one kept in shared memory (same members).
 // QUICK: the window probability from a table and the polar range from quick

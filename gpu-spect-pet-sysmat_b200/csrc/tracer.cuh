@@ -407,26 +407,4 @@ SM_HD int hole_filter(float px, float py, float pz, float dx, float dy, float dz
     return 1;
 }
 
-// Conservative culling: can any segment from a point of box A to a point of
-// box B meet box K?  K must already be inflated by the safety margin.  Uses
-// the depth (y) ordering of the scanner: at depth y a segment a -> b sits at
-// lateral position a + (b - a) * lambda, lambda = (y - a_y) / (b_y - a_y);
-// lambda is monotone in y, a_y and b_y, so its range over K's depth band comes
-// from box corners.  Returns true whenever the ordering assumption fails.
-__device__ __forceinline__ bool window_hit(const Box3& A, const Box3& B, const Box3& K) {
-    if (K.y1 > fmaxf(A.y2, B.y2) || K.y2 < fminf(A.y1, B.y1)) return false;   // K outside every segment's depth range
-    if (!(A.y2 < K.y1) || !(A.y2 < B.y1)) return true;
-    float yhi = fminf(K.y2, B.y2);
-    float lmin = (K.y1 - A.y2) / (B.y2 - A.y2);
-    float lmax = fminf(1.0f, (yhi - A.y1) / (B.y1 - A.y1));
-    lmin = fmaxf(lmin, 0.0f);
-    float xa = A.x1 + (B.x1 - A.x1) * lmin, xb = A.x1 + (B.x1 - A.x1) * lmax;
-    float xc = A.x2 + (B.x2 - A.x2) * lmin, xd = A.x2 + (B.x2 - A.x2) * lmax;
-    if (fminf(xa, xb) > K.x2 || fmaxf(xc, xd) < K.x1) return false;
-    float za = A.z1 + (B.z1 - A.z1) * lmin, zb = A.z1 + (B.z1 - A.z1) * lmax;
-    float zc = A.z2 + (B.z2 - A.z2) * lmin, zd = A.z2 + (B.z2 - A.z2) * lmax;
-    if (fminf(za, zb) > K.z2 || fmaxf(zc, zd) < K.z1) return false;
-    return true;
-}
-
 }  // namespace smb
