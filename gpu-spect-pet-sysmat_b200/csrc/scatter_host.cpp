@@ -196,8 +196,13 @@ int build_scatter_tables(const HostGeometry& g, const int sp[3], HostScatterTabl
     for (int a = 0; a < 3; ++a) s2 += (hi[a] - lo[a]) * (hi[a] - lo[a]);
     T.chord_delta = 1.5e-6f * std::sqrt(s2);
     build_kn_table(g.physics[7], &T.kn, &T.kn_inv_norm);
-    T.window.resize(kWindowNodes);
-    build_window_table(T.window.data());
+    // constants of the library: built once, 20 us
+    static const std::vector<float4> window = [] {
+        std::vector<float4> w(kWindowNodes);
+        build_window_table(w.data());
+        return w;
+    }();
+    T.window = window;
     return SM_OK;
 }
 

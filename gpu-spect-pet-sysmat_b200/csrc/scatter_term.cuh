@@ -110,11 +110,11 @@ inline void build_window_table(float4* out) {
     out[kWindowNodes - 1] = taylor_node(0.5 * std::sqrt(M_PI) * kErfSlope, 0.0, 0.0, 0.0);
 }
 
+constexpr float kErfcEnd = (float)kErfcHalf / (float)kErfcPerUnit;
+
 // The function whose node at zero is *centre, nodes to either side as far as z reaches, as the
 // node's value (x) and what is added to it (y).
 SM_HD float2 taylor_at(const float4* centre, float z) {
-    constexpr float kEnd = (float)kErfcHalf / (float)kErfcPerUnit;
-    z = fminf(fmaxf(z, -kEnd), kEnd);
     // adding 1.5 2^23 rounds to a whole number, whose low bits are the sum's
     const float magic = 12582912.0f, y = fmaf(z, (float)kErfcPerUnit, magic), k = y - magic;
 #ifdef __CUDA_ARCH__
@@ -133,28 +133,23 @@ SM_HD float2 taylor_at(const float4* centre, float z) {
 }
 
 SM_HD float erfc_at(const float4* nodes, float z) {
-    const float2 v = taylor_at(nodes + kErfcHalf, z);
+    const float2 v = taylor_at(nodes + kErfcHalf, fminf(fmaxf(z, -kErfcEnd), kErfcEnd));
     return v.x + v.y;
 }
 
 // 0.5 (erf(z2) - erf(z1)) from the table of build_window_table, without a difference of
-// rounded numbers: through erf of both sides where zero lies between the ends, else through
-// erfc of the distances, and always with the nodes' values apart from what is added to them.
+// rounded numbers: through erf of both distances where zero lies between the ends, else through
+// erfc of them, and always with the nodes' values apart from what is added to them.
 // On the GPU against double, windows of +-10 % down to +-0.05 % of the energy at 10 %
 // resolution: 4e-8 in the mean square and 2.8e-7 at most; erff and erfcf give 7e-8 and 3e-7
 // for the widest, 4e-6 and 2e-5 for the narrowest.
 SM_HD float window_probability(const float4* nodes, float z1, float z2) {
-    const bool across = z1 <= 0.0f && z2 >= 0.0f;
-    float a = z2, b = z1;
-    if (across) b = -z1;
-    else if (z2 < 0.0f) {
-        a = -z1;
-        b = -z2;
-    }
+    const bool across = (z1 < 0.0f) != (z2 < 0.0f);
     const float4* centre = nodes + (across ? kErfcNodes : kErfcHalf);
-    const float2 va = taylor_at(centre, a), vb = taylor_at(centre, b);
+    const float2 a = taylor_at(centre, fminf(fabsf(z1), kErfcEnd)), b = taylor_at(centre, fminf(fabsf(z2), kErfcEnd));
     const float sign = across ? 1.0f : -1.0f, half = across ? kErfHalf : 0.5f;
-    return fmaf(half, fmaf(sign, va.x, vb.x), half * fmaf(sign, va.y, vb.y));   // large and small parts apart
+    const float p = fmaf(half, fmaf(sign, b.x, a.x), half * fmaf(sign, b.y, a.y));   // large and small parts apart
+    return copysignf(p, z2 - z1);   // left of zero p is the difference the other way round
 }
 
 // angle between u and e (atan2 of |u x e| and u . e: accurate at every angle)
@@ -169,8 +164,9 @@ SM_HD void angle_parts(float ux, float uy, float uz, const float3& e, float* sin
 // least squares on 4001 Chebyshev points; each coefficient rounded to a float in turn, from
 // the highest, and the rest fitted again): 2.3e-8 with the coefficients as written.  The
 // quotient is corrected once and pi / 2 and pi are carried to more than 24 bits, so the
-// rest is rounding.  (Not FINE, for a decision with a margin: without these two, to 3e-7.)  On the GPU 3e-8 rad in the mean square for angles to 0.8, 8e-8 to pi;
-// atan2f, which it stands for, 3e-8 and 1.1e-7.
+// rest is rounding.  (Not FINE, for a decision with a margin: without these two, to 3e-7.)
+// On the GPU 2.3e-8 rad in the mean square for angles to 0.8, 7.3e-8 to pi; atan2f, which
+// it stands for, 2.6e-8 and 1.13e-7.
 template <bool FINE = true>
 SM_HD float angle_quick(float s, float c) {
     const float a = fabsf(c), lo = fminf(s, a), hi = fmaxf(s, a);
