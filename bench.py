@@ -40,10 +40,10 @@ sys.path.insert(0, os.path.join(ROOT, "gpu-spect-pet-sysmat_b200"))
 SLAB_Z = 4
 L2_FLUSH_BYTES = 256 << 20
 # DRAM traffic of one full pe_large slab launch (6400 x 16384 entries):
-# dram__bytes_read.sum 126.68 MB + dram__bytes_write.sum 579.35 MB from one
+# dram__bytes_read.sum 46.59 MB + dram__bytes_write.sum 431.86 MB from one
 # single-pass ncu capture of pe_trace_kernel on B200.  Algorithmic bytes of the
 # same launch: 4 B per entry of output, 419.4 MB, plus 0.64 MB of tables.
-PE_LARGE_SLAB_DRAM_BYTES = 706.03e6
+PE_LARGE_SLAB_DRAM_BYTES = 478.46e6
 PE_LARGE_SLAB_ALGORITHMIC_BYTES = 4 * 6400 * 16384 + 2 * 4 * 80000
 
 # FP32 operations per unit of work, counted from the tracer's source
@@ -460,8 +460,8 @@ def run_ours(args, world, rank, local):
 
 def run_beam_metrics(block, stream, reps: int = 5):
     """sm_beam_metrics on a resident sysmat block (masks kept): HBM-bound;
-    algorithmic bytes per entry = 4 (sysmat read) + 1 (mask written) + 1
-    (mask read for MPXI).  The block (419 MB for pe_large) exceeds L2."""
+    algorithmic bytes per entry = 4 (sysmat read) + 1 (mask written).  The
+    block (419 MB for pe_large) exceeds L2."""
     import torch
     from sysmat_b200 import beams
     peaks, src = load_peaks()
@@ -479,9 +479,9 @@ def run_beam_metrics(block, stream, reps: int = 5):
     stream.synchronize()
     ms = e0.elapsed_time(e1) / reps
     entries = block.shape[0] * block.shape[1]
-    gbs = 6.0 * entries / (ms / 1e3) / 1e9
+    gbs = 5.0 * entries / (ms / 1e3) / 1e9
     hbm = float(peaks.get("hbm_gbs", 6650.0))
-    return {"entries": entries, "ms": ms, "bytes_per_entry": 6, "achieved_gbs": gbs, "peak_gbs": hbm,
+    return {"entries": entries, "ms": ms, "bytes_per_entry": 5, "achieved_gbs": gbs, "peak_gbs": hbm,
             "frac": gbs / hbm, "peak_source": src, "active_rows": int((m["row_count"] > 0).sum()),
             "mpxi_max": int(m["mpxi"].max()),
             "timed": "row stats + int8 masks + MPXI of the resident slab 0, CUDA events, mean of %d" % reps}

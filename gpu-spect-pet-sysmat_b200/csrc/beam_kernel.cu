@@ -16,8 +16,9 @@
 //                     the counts leave in one integer atomicAdd per voxel at the end,
 //                     exact and independent of order.  HBM-bound: 4 bytes read and 1
 //                     written per entry, nothing twice.  6400 x 16384 with mask and
-//                     MPXI through beam_held_kernel (its comment): 99 us, 5.3
-//                     TB/s; two passes over global memory took 171 us.
+//                     MPXI through beam_held_kernel (its comment): 99 to 108
+//                     us from one GPU to another, 4.9 to 5.3 TB/s; two passes over global
+//                     memory took 171 us.
 //  beam_rows_kernel   longer rows.  One CTA per row (grid-stride): pass A reduces max
 //                     and sum with 128-bit loads; pass B re-reads the row (from L2) and
 //                     writes the int8 mask with 32-bit stores and counts it.

@@ -19,12 +19,12 @@
 //  * the epilogue warps read 32 columns of their 32 TMEM lanes, pass them through
 //    shared memory, and store whole 128-byte rows.
 // What bounds it: for the surrogate's shapes (K = 256) the fp32 result, then the chain
-// of a tile's four chunks: 2048 x 131072 x 256 takes 215 us back to back and 257 us from a
-// flushed L2 (a plain fill of the result 144 us, the same walk storing an eighth of the
+// of a tile's four chunks: 2048 x 131072 x 256 takes 224 us back to back and 269 us on
+// inputs that are not in L2 (a plain fill of the result 144 us, the same walk storing an eighth of the
 // columns 140 us), the version before, one CTA per tile with loads, MMAs and stores in
 // turn, 2072 us.  With rows off
-// 16 bytes (1491 x 3906 x 975) 120 us against 203; both operands row-contiguous
-// (1000 x 20000 x 512) 205 us against 460.
+// 16 bytes (1491 x 3906 x 975) 110 us against 203; both operands row-contiguous
+// (1000 x 20000 x 512) 201 us against 460.
 //
 // Every wait is bounded (wait_limit polls, set process-wide by
 // sm_tc_wait_limit): a wait that runs out sets the error word, the roles stop and

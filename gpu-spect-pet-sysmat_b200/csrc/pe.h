@@ -38,7 +38,7 @@ struct PEParams {
     float cos_a, sin_a;      // image rotation about z
     int dX, dY, dZ;          // crystal sub-cells
     int n_sc, n_sv, group;   // sub-cells per crystal, sub-points per voxel, sub-points per mask group
-    int pair;                // voxels per group of sub-points (1..8): > 1 for entries of at most 64 rays (see pe_plan)
+    int pair;                // voxels per group of sub-points (1..8): > 1 for entries of few rays (see pe_plan)
     int rotated;             // some crystal is rotated
     float inv_sv;
     float chord_delta;       // half-size margin of chord_filter: 1.5e-6 of the coordinate range

@@ -549,9 +549,11 @@ __device__ __forceinline__ float trace_ray(const PEParams& P, const DevGeometry&
             len = crystal_chord_exact(p, q, kp, kh, kc, ks);
             if (len == 0.0f) return;
         } else if (FEW) {
-            // Entries of few rays keep the exact form's rounding (their matrices feed the
-            // scatter pipeline, whose bf16 operands and error estimates magnify it); entries
-            // of many rays average the filter's, which is of the same size.
+            // Entries of the few-ray form keep the exact form's rounding (their matrices feed the
+            // scatter pipeline, whose bf16 operands and error estimates magnify it).  The
+            // others' chords are the filter's: against 64 bits 1.21e-6 of an entry in the mean
+            // square (28 geometries, 24 to 3072 rays), 1.28e-6 with chord_value for all, which
+            // takes 12 to 20 % longer.
             const float ax = p.x - kp.x, az = p.z - kp.z, bx = q.x - kp.x, bz = q.z - kp.z;
             if (!ROT || !(e & kRotated))
                 len = chord_value(ax, p.y - kp.y, az, bx, q.y - kp.y, bz, kh.x, kh.y, kh.z, cr.ix, cr.iy, cr.iz, inv_r);

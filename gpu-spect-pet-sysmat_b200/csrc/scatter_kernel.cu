@@ -563,10 +563,11 @@ __global__ void __launch_bounds__(kTrRanks * kTrSrcs) scatter_transfer_tiled_ker
 //  3. whenever 32 entries wait, one term per lane; the sums are doubles in shared memory,
 //     every cell owned by one warp and added to in (source, point) order, so the split
 //     into columns, rows lists and bricks changes no bit.
-// What bounds it: instruction issue (FP32 and transcendental; 63 % of the slots taken, the
+// What bounds it: instruction issue (FP32 and transcendental; 66 % of the slots taken, the
 // rest fixed latencies), 2 CTAs of 8 warps per SM by registers and shared memory alike.
-// 2048 detectors x 16384 voxels x 2048 points: 224 ms with the terms evaluated where their
-// lane is the detector (17 of 32 lanes at work), 136 ms in this form.
+// 2048 detectors x 16384 voxels x 2048 points, the whole call with its pairs: 297 ms with
+// the terms evaluated where their lane is the detector (17 of 32 lanes at work), 140 ms in
+// this form.
 template <int C>
 struct ScShape {
     static constexpr int NQ = 8;                       // points per batch (shared memory: 5 KB each)
